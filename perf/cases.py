@@ -277,3 +277,76 @@ def tolerance(case):
         return {"rel": 8e-4, "max": 0.15}
     # chained, so that steps of the quantised intermediate values reach the outputs too: 1.7e-4
     return {"rel": 1e-3, "max": 0.15}
+
+
+# ----------------------------------------------------------- 64-bit values ---
+
+def _quant64(y, block_rows=1):
+    """Values of the block quantisation as float64: (q, scale), block_rows x 128 blocks, q rounded to e4m3."""
+    R, C = y.shape
+    b = y.view(R // block_rows, block_rows, C // 128, 128)
+    s = b.abs().amax(dim=(1, 3)) / 448.0
+    q = torch.where(s[:, None, :, None] > 0, b / s[:, None, :, None], torch.zeros_like(b))
+    return q.view(R, C).float().to(torch.float8_e4m3fn).double(), s
+
+
+def _quant32(x, block_rows=1):
+    """The quantised operands that `prepare` makes (IEEE fp32 divisions), de-quantised to float64."""
+    R, C = x.shape
+    b = x.view(R // block_rows, block_rows, C // 128, 128)
+    s = b.abs().amax(dim=(1, 3), keepdim=True) / torch.tensor(448.0, device=x.device)
+    q = torch.where(s > 0, b / s, torch.zeros_like(b)).to(torch.float8_e4m3fn)
+    return (q.double() * s.double()).view(R, C)
+
+
+def _out64(y):
+    """(e4m3 values, [N/128, M] scales) of an e4m3 output."""
+    q, s = _quant64(y)
+    return q, s.t().contiguous()
+
+
+def _deq64(y):
+    q, s = _quant64(y)
+    return q * s.repeat_interleave(128, dim=1)
+
+
+def _rms64(x, w):
+    return x / torch.sqrt((x * x).mean(dim=-1, keepdim=True) + EPS) * w
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind == "weights":
+        return None  # bytes: compared exactly
+    g, M = _gen(seed), case["M"]
+    if kind == "fp16_mm":
+        dt = getattr(torch, case["dtype"])
+        A = torch.rand(M, case["K"], generator=g, device="cuda").mul_(2).sub_(1).to(dt)
+        B = torch.rand(case["K"], case["N"], generator=g, device="cuda").mul_(2).sub_(1).to(dt)
+        return A.double() @ B.double()
+    if kind == "fp8_mm":
+        A = _quant32(_normal(g, M, case["K"]))
+        B = _quant32(_normal(g, case["N"], case["K"], std=0.02), 128)
+        return _out64(A @ B.t()) if case["out"] == "e4m3" else A @ B.t()
+    shapes = _shapes(case)
+    if kind in ("linears", "mlp"):
+        A = [_quant32(_normal(g, M, K)) for _, K in shapes]
+        B = [_quant32(_normal(g, N, K, std=0.02), 128) for N, K in shapes]
+        return [_out64(a @ b.t()) for a, b in zip(A, B)]
+    H, I, n_q, n_kv = case["hidden"], case["inter"], case["q_heads"], case["kv_heads"]
+    x, attn = _normal(g, M, H).double(), _normal(g, M, n_q * 128)
+    w_in, w_post, w_q, w_k = [_normal(g, n, std=0.1).add_(1.0).double() for n in (H, H, 128, 128)]
+    angle = torch.outer(torch.arange(TABLE_ROWS, device="cuda", dtype=torch.float32),
+                        1e6 ** (-torch.arange(64, device="cuda", dtype=torch.float32) / 64))
+    pos = torch.randint(0, TABLE_ROWS, (M,), generator=g, device="cuda", dtype=torch.int32).long()
+    cos, sin = angle.cos()[pos].double()[:, None], angle.sin()[pos].double()[:, None]
+    w_qkv, w_o, w_gate_up, w_down = [_quant32(_normal(g, N, K, std=0.02), 128) for N, K in shapes]
+    qkv = (_deq64(_rms64(x, w_in)) @ w_qkv.t()).view(M, -1, 128)
+    for lo, hi, w in ((0, n_q, w_q), (n_q, n_q + n_kv, w_k)):
+        h = _rms64(qkv[:, lo:hi], w)
+        a, b = h[..., :64], h[..., 64:]
+        qkv[:, lo:hi] = torch.cat([a * cos - b * sin, b * cos + a * sin], dim=2)
+    o = _quant32(attn) @ w_o.t()
+    acc = _deq64(_rms64(o, w_post)) @ w_gate_up.t()
+    h = acc[:, :I] / (1 + torch.exp(-acc[:, :I])) * acc[:, I:]
+    return {"qkv": _out64(qkv.reshape(M, -1)), "o": o, "h": _out64(h), "y": _deq64(h) @ w_down.t()}
