@@ -32,6 +32,7 @@
 //     the tile leaves as whole rows (a thread storing its own row would make
 //     every store instruction of the warp touch 32 rows); the scale column is
 //     stored directly, it is coalesced.
+#include <cstddef>
 #include <cuda_fp8.h>
 
 #include "host_common.h"
@@ -400,44 +401,40 @@ constexpr int      BM         = 256;  // per pair; 128 rows per CTA
 constexpr int      BN         = 256;
 constexpr int      BK         = 128;
 constexpr int      UMMA_K     = 32;
-constexpr int      STAGES     = 6;
 constexpr int      THREADS    = 384;
-constexpr int      REGS_CTRL  = 32;  // 32/232 compiles without spills; 40/232 spilt in the promotion loop (+35 % time)
+constexpr int      REGS_CTRL  = 40;  // (32 spilt in the promotion loop)
 constexpr int      REGS_PROMO = 232;
 static_assert(128 * REGS_CTRL + 256 * REGS_PROMO <= THREADS * 168, "setmaxnreg split exceeds the CTA's registers");
 constexpr uint32_t A_BYTES    = 128 * BK;                 // 16 KB: this CTA's rows
 constexpr uint32_t B_BYTES    = 128 * BK;                 // 16 KB: this CTA's half of the tile's columns
 constexpr uint32_t STAGE_TX   = 2 * (A_BYTES + B_BYTES);  // both CTAs' loads land on the leader's barrier
-constexpr uint32_t OFF_A      = 0;
-constexpr uint32_t OFF_B      = OFF_A + STAGES * A_BYTES;
-constexpr uint32_t OFF_BAR    = OFF_B + STAGES * B_BYTES;
-constexpr uint32_t OFF_XCH    = OFF_BAR + 256;  // 2 x 256 floats: row maxima exchanged between the column halves (SWIGLU)
-// The e4m3 epilogues transpose each promotion warp's 32 x 128-byte output tile through 4 KB of shared memory
-// (16-byte chunks XOR-swizzled by row, which is the 128-byte swizzle of a tensor map), so that the tile leaves as
-// whole rows: one TMA store per warp (EPI_E4M3) or store instructions that cover four rows each.  EPI_E4M3 and
-// EPI_GATHER keep the eight staging tiles from OFF_STG on (1024-byte aligned; SWIGLU's exchange buffer overlaps
-// it, that instantiation has no staging tiles).
-constexpr uint32_t OFF_STG           = OFF_BAR + 1024;
-constexpr uint32_t SMEM_BYTES_STAGED = OFF_STG + 8 * 4096 + 1024;
-static_assert(SMEM_BYTES_STAGED <= 232448, "staging tiles + ring exceed the shared memory of an SM");
-// EPI_ROPE keeps the angle-table rows of the tile's 128 rows in shared memory: 32 rows x (256 B cos | 256 B sin)
-// = 16 KB per row quarter.  Quarters 0 and 1 use the two slots of the ring's sixth stage (the ring runs with
-// five), quarters 2 and 3 the 32 KB from OFF_STG on; the two norm weight vectors follow.  Once a tile's rows have
-// been used, the first 8 KB of each quarter's region serve as the two staging tiles of its warps.
-constexpr uint32_t ROPE_TAB_BYTES  = 32 * 512;
-constexpr uint32_t OFF_ROPE_W      = OFF_STG + 2 * ROPE_TAB_BYTES;  // 2 x 128 floats: query and key norm weights
-constexpr uint32_t SMEM_BYTES_ROPE = OFF_ROPE_W + 1024 + 1024;
-
-// EPI_SWIGLU: a warp's output tile is 32 rows x 64 bytes (2 KB, 16-byte chunks in the 64-byte swizzle of a tensor
-// map); its eight staging tiles lie behind the exchange buffer.
-constexpr uint32_t OFF_STG_SWIGLU    = OFF_BAR + 3072;
-constexpr uint32_t SMEM_BYTES_SWIGLU = OFF_STG_SWIGLU + 8 * 2048 + 1024;
-static_assert(OFF_XCH + 2048 <= OFF_STG_SWIGLU, "exchange buffer and staging tiles overlap");
-
-constexpr uint32_t smem_bytes_of(int epi)  // (the EPI_* constants: 2 swiglu, 4 rope)
-{
-  return epi == 4 ? SMEM_BYTES_ROPE : epi == 2 ? SMEM_BYTES_SWIGLU : SMEM_BYTES_STAGED;
-}
+// Ring of scale operands, filled by a warp of its own: a slot holds SC_KB K-blocks of this CTA's 128 A scales
+// followed by the tile's two B scales (SWIGLU: the gate rows' and the up rows').
+constexpr int      SC_KB      = 4;
+constexpr int      SC_SLOTS   = 4;
+constexpr int      SC_ROW     = 132;  // floats per K-block: 128 + 2, padded to 16 bytes
+constexpr uint32_t SC_BYTES   = SC_SLOTS * SC_KB * SC_ROW * 4;
+// Shared memory, per epilogue (the EPI_* constants: 2 swiglu, 4 rope): operand ring | barriers | scale ring |
+// what the epilogue needs.
+//   EPI_E4M3 / EPI_F32 / EPI_GATHER: eight 4 KB staging tiles.  Each promotion warp transposes its 32 x 128-byte
+//     output tile through one (16-byte chunks XOR-swizzled by row, which is the 128-byte swizzle of a tensor map),
+//     so that the tile leaves as whole rows: one TMA store per warp or store instructions that cover four rows each.
+//   EPI_SWIGLU: 2 x 256 floats in which the column halves exchange row maxima, and eight 2 KB staging tiles (32
+//     rows x 64 bytes, 64-byte swizzle).
+//   EPI_ROPE: the angle-table rows of the tile's 128 rows, 32 rows x (256 B cos | 256 B sin) = 16 KB per row
+//     quarter, then the two norm weight vectors.  Once a tile's rows have been used, the first 8 KB of each
+//     quarter's region serve as the two staging tiles of its warps.
+constexpr uint32_t ROPE_TAB_BYTES = 32 * 512;
+__host__ __device__ constexpr uint32_t nstages(int epi) { return epi == 4 ? 4 : epi == 2 ? 6 : 5; }
+__host__ __device__ constexpr uint32_t off_b(int epi) { return nstages(epi) * A_BYTES; }
+__host__ __device__ constexpr uint32_t off_stg(int epi) { return nstages(epi) * (A_BYTES + B_BYTES); }  // 1024-byte aligned
+__host__ __device__ constexpr uint32_t stg_bytes(int epi) { return epi == 4 ? 4 * ROPE_TAB_BYTES : epi == 2 ? 8 * 2048 : 8 * 4096; }
+__host__ __device__ constexpr uint32_t off_xch(int epi) { return off_stg(epi) + stg_bytes(epi); }  // SWIGLU: row maxima, ROPE: norm weights
+__host__ __device__ constexpr uint32_t xch_bytes(int epi) { return epi == 4 ? 1024 : epi == 2 ? 2048 : 0; }
+__host__ __device__ constexpr uint32_t off_sc(int epi) { return off_xch(epi) + xch_bytes(epi); }
+__host__ __device__ constexpr uint32_t off_bar(int epi) { return off_sc(epi) + SC_BYTES; }
+__host__ __device__ constexpr uint32_t smem_bytes_of(int epi) { return off_bar(epi) + 512 + 1024; }
+static_assert(smem_bytes_of(0) <= 232448 && smem_bytes_of(2) <= 232448 && smem_bytes_of(4) <= 232448, "shared memory of an SM");
 constexpr uint32_t TMEM_COLS  = 512;  // two partial stages of 256 columns
 // split tiles (pair_walk.cuh): a slot holds 16 warp-sized units of 32 rows x 128 columns
 constexpr size_t   SK_UNIT_FLOATS = 32 * 128;
@@ -445,10 +442,12 @@ static_assert(16 * SK_UNIT_FLOATS == SPLIT_SLOT_FLOATS, "one slot per 256x256 ti
 }  // namespace fp8pair
 
 struct Fp8PairBars {
-  uint64_t full[fp8pair::STAGES];   // used in the leader CTA
-  uint64_t empty[fp8pair::STAGES];  // both CTAs (multicast commit)
-  uint64_t part_full[2];            // both CTAs (multicast commit)
-  uint64_t part_empty[2];           // used in the leader CTA, 16 arrivals
+  uint64_t full[6];        // used in the leader CTA
+  uint64_t done[6];        // both CTAs (multicast commit): the K-block's MMAs are done, so the ring slot is free and
+                           // the partial stage can be read (one commit per K-block serves both)
+  uint64_t part_empty[2];  // used in the leader CTA, 16 arrivals
+  uint64_t sc_full[fp8pair::SC_SLOTS];   // 32 arrivals: the scale warp's lanes, when their copies have landed
+  uint64_t sc_empty[fp8pair::SC_SLOTS];  // 8 arrivals: the promotion warps
   uint32_t tmem_base;
   uint32_t abort_flag;
 };
@@ -528,6 +527,13 @@ __device__ __forceinline__ float4 ldg_pinned(const float4* p)
   return v;
 }
 
+__device__ __forceinline__ float lds_f32(uint32_t addr)
+{
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+
 // the same for shared memory
 __device__ __forceinline__ float4 lds_pinned(uint32_t addr)
 {
@@ -540,6 +546,18 @@ __device__ __forceinline__ float4 lds_pinned(uint32_t addr)
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src)
 {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// 4 bytes (both addresses 4-byte aligned)
+__device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// One of the barrier's expected arrivals, when all copies of this thread so far have landed.
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar)
+{
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ void cp_async_wait_all()
@@ -573,11 +591,12 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
   constexpr bool OUT_F32 = (EPI == EPI_F32);
   constexpr bool SWIGLU  = (EPI == EPI_SWIGLU);
   constexpr int  TILE_N  = SWIGLU ? 128 : BN;  // output columns per tile
-  // EPI_ROPE runs the ring one stage shorter: the sixth stage's two 16 KB slots hold angle-table rows
-  constexpr uint32_t NSTAGES = EPI == EPI_ROPE ? STAGES - 1 : STAGES;
+  constexpr uint32_t NSTAGES = nstages(EPI);
+  constexpr uint32_t OFF_A = 0, OFF_B = off_b(EPI), OFF_STG = off_stg(EPI), OFF_XCH = off_xch(EPI);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  Fp8PairBars*       bars       = reinterpret_cast<Fp8PairBars*>(smem + OFF_BAR);
+  Fp8PairBars*       bars       = reinterpret_cast<Fp8PairBars*>(smem + off_bar(EPI));
+  float*             sc_ring    = reinterpret_cast<float*>(smem + off_sc(EPI));
   volatile uint32_t* abort_flag = &bars->abort_flag;
 
   const int      warp    = threadIdx.x >> 5;
@@ -591,13 +610,16 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
   const int n_groups = N / 128;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (uint32_t s = 0; s < NSTAGES; ++s) {
       mbar_init(&bars->full[s], 1);
-      mbar_init(&bars->empty[s], 1);
+      mbar_init(&bars->done[s], 1);
     }
     for (int p = 0; p < 2; ++p) {
-      mbar_init(&bars->part_full[p], 1);
       mbar_init(&bars->part_empty[p], 16);  // 8 promotion warps of each CTA
+    }
+    for (int i = 0; i < SC_SLOTS; ++i) {
+      mbar_init(&bars->sc_full[i], 32);
+      mbar_init(&bars->sc_empty[i], 8);
     }
     bars->abort_flag = 0;
     fence_mbar_init();
@@ -633,7 +655,7 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
           for (int kb = kb0; kb < kb1; ++kb, ++it) {
             const uint32_t s  = it % NSTAGES;
             const uint32_t ph = (it / NSTAGES) & 1;
-            mbar_wait(&bars->empty[s], ph ^ 1, DEV_WAIT_SMEM_EMPTY, abort_flag, status);
+            mbar_wait(&bars->done[s], ph ^ 1, DEV_WAIT_SMEM_EMPTY, abort_flag, status);
             const uint32_t full_leader = mapa_shared(smem_u32(&bars->full[s]), 0);
             if (rank == 0) {
               mbar_arrive_expect_tx(&bars->full[s], STAGE_TX);
@@ -651,7 +673,43 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
         }
       }
     }
-    else if (warp == 1 || warp == 3) {
+    else if (warp == 2) {
+      // ---------------------------------------------------- scale operands --
+      // The promotion warps must never wait for global memory: the slowest of the 16 warps of a pair decides when a
+      // partial stage can be written again, and under the operand traffic an L2 hit takes one to two K-blocks.  This
+      // warp therefore copies the scales up to SC_SLOTS * SC_KB K-blocks ahead.  (Copies of 4 bytes: a row of A_s
+      // starts at a multiple of 16 bytes only if M is a multiple of 4.)  While every promotion thread fetched its own
+      // scales two K-blocks ahead, a K-block took 1078 clk at 4096^3 and 1458 clk at 8192x4096x8192; with the ring
+      // (and one commit per K-block instead of two) 943 and 911.
+      uint32_t c = 0;
+      PairWalk walk(pair, n_pairs, k_blocks, dp_tiles, split_pairs, split_s, split_chunk);
+      int      tile, kb0, kb1;
+      while (walk.next(tile, kb0, kb1)) {
+        const int m0 = (tile % m_tiles) * BM + (int)rank * 128 + lane;
+        const int g  = SWIGLU ? tile / m_tiles + (lane & 1) * n_groups : (tile / m_tiles) * (BN / 128) + (lane & 1);
+        // (rows and groups beyond the matrix read valid scales of others: their results are not stored)
+        const float* b_s = B_s + (size_t)(SWIGLU || g < n_groups ? g : 0) * k_blocks;
+        for (int kb = kb0; kb < kb1; kb += SC_KB, ++c) {
+          const uint32_t slot = c % SC_SLOTS;
+          mbar_wait(&bars->sc_empty[slot], ((c / SC_SLOTS) & 1) ^ 1, DEV_WAIT_SMEM_EMPTY, abort_flag, status);
+          uint32_t dst = smem_u32(sc_ring) + (slot * SC_KB * SC_ROW + lane) * 4;
+#pragma unroll 1
+          for (int k = kb; k < min(kb + SC_KB, kb1); ++k, dst += SC_ROW * 4) {
+            const float* a_s = A_s + (size_t)k * M;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              cp_async_4(dst + i * 128, a_s + min(m0 + 32 * i, M - 1));
+            }
+            if (lane < 2) {
+              cp_async_4(dst + 512, b_s + k);
+            }
+          }
+          cp_async_arrive(&bars->sc_full[slot]);
+        }
+      }
+      cp_async_wait_all();
+    }
+    else {
       // ------------------------------------ two MMA issuers (leader only) --
       // A thread that issues a group of MMAs followed by tcgen05.commit is held for about the
       // duration of the group (measured: one thread feeds the pipe at 160-190 clk per MMA, two
@@ -693,8 +751,7 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
             for (int kk = 0; kk < BK / UMMA_K; ++kk) {
               tc_mma_f8_pair(tmem_base + p * BN, da + (uint64_t)((kk * UMMA_K) >> 4), db + (uint64_t)((kk * UMMA_K) >> 4), idesc, kk != 0);
             }
-            tc_commit_pair(&bars->empty[s]);
-            tc_commit_pair(&bars->part_full[p]);
+            tc_commit_pair(&bars->done[s]);
 #ifdef LLMMM_PROFILE
             if (blockIdx.x == 0 && it < 64) {
               g_trace8[it][3] = clock64();  // MMAs and commits issued
@@ -722,21 +779,24 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
 #endif
     const int      quarter = warp & 3;         // TMEM lane quarter this warp may read
     const int      half    = (warp - 4) >> 2;  // which 128-column scale group of the tile
-    const uint32_t t_lane  = ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
-    const uint32_t empty_leader[2] = {mapa_shared(smem_u32(&bars->part_empty[0]), 0),
-                                      mapa_shared(smem_u32(&bars->part_empty[1]), 0)};
-    uint32_t it = 0;
+    const uint32_t t_mine  = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);  // this warp's part of stage 0
+    // (barriers are addressed by 32-bit shared-memory addresses: the loop has no register to spare)
+    const uint32_t bars_at      = smem_u32(bars);
+    const uint32_t abort_at     = smem_u32(&bars->abort_flag);
+    const uint32_t empty_leader = mapa_shared(smem_u32(&bars->part_empty[0]), 0);
+    uint32_t       it           = 0;
+    uint32_t       done_at = bars_at + (uint32_t)offsetof(Fp8PairBars, done), done_ph = 0;  // of K-block `it`
+    uint32_t       sc_slot = 0, sc_ph = 0;
+    const uint32_t sc_mine = smem_u32(sc_ring) + (quarter * 32 + lane) * 4;  // this thread's row in slot 0 ...
+    const uint32_t sc_b    = (128 - quarter * 32 - lane + (SWIGLU ? 0 : half)) * 4;  // ... and from there to its B scale
     PairWalk walk(pair, n_pairs, k_blocks, dp_tiles, split_pairs, split_s, split_chunk);
     int      tile, kb_lo, kb_hi;
     uint32_t tile_count = 0;  // SWIGLU: which exchange buffer
     // EPI_ROPE: where this warp's row quarter keeps its angle-table rows (32 rows x 512 B, 16-byte chunks
     // XOR-swizzled by row), shared by the two warps of the quarter, and the staged norm weights
-    const uint32_t rope_off = EPI != EPI_ROPE ? 0u
-                              : quarter == 0  ? OFF_A + (STAGES - 1) * A_BYTES
-                              : quarter == 1  ? OFF_B + (STAGES - 1) * B_BYTES
-                                              : OFF_STG + (quarter - 2) * ROPE_TAB_BYTES;
+    const uint32_t rope_off = EPI != EPI_ROPE ? 0u : OFF_STG + quarter * ROPE_TAB_BYTES;
     const uint32_t rope_tab = smem_u32(smem + rope_off);
-    const uint32_t rope_w   = smem_u32(smem + OFF_ROPE_W);
+    const uint32_t rope_w   = smem_u32(smem + OFF_XCH);
     // position of this lane's output row in tile t (rows beyond M use the first position); only the load is
     // issued here, the value is looked at a main loop later
     auto rope_row = [=](int t) -> int {
@@ -766,7 +826,7 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
       // the norm weights (ones without a weight vector: one straight line of arithmetic either way)
       const int    t    = (int)threadIdx.x - 128;
       const float* wsrc = t < 128 ? rope.q_w : rope.k_w;
-      reinterpret_cast<float*>(smem + OFF_ROPE_W)[t] = wsrc != nullptr ? __ldg(wsrc + (t & 127)) : 1.0f;
+      reinterpret_cast<float*>(smem + OFF_XCH)[t] = wsrc != nullptr ? __ldg(wsrc + (t & 127)) : 1.0f;
       asm volatile("bar.sync 1, 256;" ::: "memory");
       if (pair < dp_tiles && rope_rotated(pair)) {
         rope_stage(rope_row(pair));
@@ -781,61 +841,25 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
           rope_p_next = rope_row(tile + n_pairs);
         }
       }
-      const int  m    = (tile % m_tiles) * BM + (int)rank * 128 + quarter * 32 + lane;
-      // global 128-column group of the output (and, except for SWIGLU, of the weight scales)
-      const int  ng   = SWIGLU ? tile / m_tiles : (tile / m_tiles) * (BN / 128) + half;
-      const bool m_ok = m < M;
-      const bool g_ok = ng < n_groups;
-      const float* a_s = A_s + (m_ok ? m : 0);
-      const float* b_s = B_s + (size_t)(g_ok ? ng : 0) * k_blocks;               // SWIGLU: the gate rows' scales
-      const float* b_up = B_s + (size_t)(n_groups + (g_ok ? ng : 0)) * k_blocks;  // SWIGLU only: the up rows' scales
-
       float acc[128];
 #pragma unroll
       for (int i = 0; i < 128; ++i) {
         acc[i] = 0.0f;
       }
 
-      // scale operands are fetched PREFETCH K-blocks ahead (an L2 hit under the TMA traffic takes
-      // longer than one K-block); the empty asm pins their first use to their own iteration
-      constexpr int PREFETCH = 2;
-      float         a_pf[PREFETCH], b_pf[PREFETCH], b2_pf[PREFETCH];
-#pragma unroll
-      for (int j = 0; j < PREFETCH; ++j) {
-        a_pf[j] = (kb_lo + j < kb_hi) ? __ldg(a_s + (size_t)(kb_lo + j) * M) : 0.0f;
-        b_pf[j] = (kb_lo + j < kb_hi) ? __ldg(b_s + kb_lo + j) : 0.0f;
-        if constexpr (SWIGLU) {
-          b2_pf[j] = (kb_lo + j < kb_hi) ? __ldg(b_up + kb_lo + j) : 0.0f;
-        }
-      }
-      for (int kb0 = kb_lo; kb0 < kb_hi; kb0 += PREFETCH) {
-#pragma unroll
-        for (int j = 0; j < PREFETCH; ++j) {
-          const int kb = kb0 + j;
-          if (kb >= kb_hi) {
-            break;
-          }
-          const uint32_t p  = it & 1;
-          const uint32_t pp = (it >> 1) & 1;
-          float a_cur = a_pf[j], b_cur = b_pf[j];
-          asm volatile("" : "+f"(a_cur), "+f"(b_cur));
+      for (int left = kb_hi - kb_lo; left > 0; left -= SC_KB) {
+        mbar_wait_at(bars_at + (uint32_t)offsetof(Fp8PairBars, sc_full) + sc_slot * 8, sc_ph, DEV_WAIT_SMEM_FULL, abort_at, status);
+        uint32_t       sc_addr = sc_mine + sc_slot * (SC_KB * SC_ROW * 4);
+        const uint32_t sc_end  = sc_addr + min(left, SC_KB) * (SC_ROW * 4);
+#pragma unroll 1
+        for (; sc_addr != sc_end; sc_addr += SC_ROW * 4) {
+          const uint32_t p = it & 1;
           // one fp32 rounding of the scale product, as in the reference
-          const float sc2 = __fmul_rn(a_cur, b_cur);
-          float       sc2_late = sc2;  // the scale of the last 64 accumulators: the up rows' for SWIGLU
-          if constexpr (SWIGLU) {
-            float b2_cur = b2_pf[j];
-            asm volatile("" : "+f"(b2_cur));
-            sc2_late = __fmul_rn(a_cur, b2_cur);
-          }
-          if (kb + PREFETCH < kb_hi) {
-            a_pf[j] = __ldg(a_s + (size_t)(kb + PREFETCH) * M);
-            b_pf[j] = __ldg(b_s + kb + PREFETCH);
-            if constexpr (SWIGLU) {
-              b2_pf[j] = __ldg(b_up + kb + PREFETCH);
-            }
-          }
+          const float a_cur    = lds_f32(sc_addr);
+          const float sc2      = __fmul_rn(a_cur, lds_f32(sc_addr + sc_b));
+          float       sc2_late = SWIGLU ? __fmul_rn(a_cur, lds_f32(sc_addr + sc_b + 4)) : sc2;  // of the last 64 accumulators (SWIGLU: the up rows')
           PROF8_T(d0);
-          mbar_wait(&bars->part_full[p], pp, DEV_WAIT_TMEM_FULL, abort_flag, status);
+          mbar_wait_at(done_at, done_ph, DEV_WAIT_TMEM_FULL, abort_at, status);
           PROF8_T(d1);
           PROF8_ADD(p_wait, d0, d1);
 #ifdef LLMMM_PROFILE
@@ -845,7 +869,7 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
           }
 #endif
           tc_fence_after_sync();
-          const uint32_t t_addr = tmem_base + p * BN + t_lane;
+          const uint32_t t_addr = t_mine + p * BN;
           // two loads in flight; the partial stage is handed back as early as possible
           uint32_t v0[32], v1[32];
           tmem_ld_32x32b_x32(t_addr, v0);
@@ -866,12 +890,7 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) {
-            if (rank == 0) {
-              mbar_arrive(&bars->part_empty[p]);
-            }
-            else {
-              mbar_arrive_cluster_relaxed(empty_leader[p]);
-            }
+            mbar_arrive_cluster_relaxed(empty_leader + p * 8);
           }
 #ifdef LLMMM_PROFILE
           if (blockIdx.x == 0 && threadIdx.x == 128 && it < 64) {
@@ -891,10 +910,27 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
             ffma2(acc[96 + i], acc[96 + i + 1], v1[i], v1[i + 1], sc2_late);
           }
           ++it;
+          done_at += 8;
+          if (done_at == bars_at + (uint32_t)offsetof(Fp8PairBars, done) + NSTAGES * 8) {
+            done_at -= NSTAGES * 8;
+            done_ph ^= 1;
+          }
+        }
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive_at(bars_at + (uint32_t)offsetof(Fp8PairBars, sc_empty) + sc_slot * 8);
+        }
+        if (++sc_slot == SC_SLOTS) {
+          sc_slot = 0;
+          sc_ph ^= 1;
         }
       }
 
       PROF8_T(e0);
+      const int  m    = (tile % m_tiles) * BM + (int)rank * 128 + quarter * 32 + lane;
+      const int  ng   = SWIGLU ? tile / m_tiles : (tile / m_tiles) * (BN / 128) + half;  // 128-column group of the output
+      const bool m_ok = m < M;
+      const bool g_ok = ng < n_groups;
       if (!SWIGLU && EPI != EPI_ROPE && kb_hi - kb_lo < k_blocks) {  // (SWIGLU and ROPE tiles are never cut)
         // A chunk of a split tile, the last piece of work of this pair.  This warp's 32x128 piece is handled
         // independently of the other warps: publish the partial sum (four columns per lane side by side:
@@ -1040,7 +1076,7 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
         amax = fmaxf(amax, xch[(half ^ 1) * 128 + quarter * 32 + lane]);
         // The warp's 32 x 64 output bytes go through a staging tile and leave as one TMA store (whole rows instead
         // of 16-byte pieces in 32 rows per store instruction); all lanes take part, rows beyond M are clipped.
-        uint8_t* stg = smem + OFF_STG_SWIGLU + (warp - 4) * 2048;
+        uint8_t* stg = smem + OFF_STG + (warp - 4) * 2048;
         if (lane == 0) {
           tma_store_wait_read<0>();  // the store of the previous tile has read the staging tile
         }
@@ -1291,7 +1327,7 @@ static int launch_fp8_swiglu(const void*       A,
   static thread_local bool attr_set[64] = {};
   if (!attr_set[info->device]) {
     LLMMM_CUDA_TRY(cudaFuncSetAttribute(
-      fp8_blockwise_gemm_pair_kernel<EPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES_SWIGLU));
+      fp8_blockwise_gemm_pair_kernel<EPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes_of(EPI_SWIGLU)));
     attr_set[info->device] = true;
   }
   // a tile is 256 rows x 128 output columns (128 gate + 128 up weight rows); tiles are never cut along K here:
@@ -1300,7 +1336,7 @@ static int launch_fp8_swiglu(const void*       A,
   const int pairs = tiles < info->max_pairs ? tiles : info->max_pairs;
   float*    no_partials = nullptr;
   uint32_t* no_counters = nullptr;
-  LLMMM_CUDA_TRY(launch_pdl(fp8_blockwise_gemm_pair_kernel<EPI_SWIGLU>, dim3(2 * pairs), dim3(THREADS), SMEM_BYTES_SWIGLU, stream, 2,
+  LLMMM_CUDA_TRY(launch_pdl(fp8_blockwise_gemm_pair_kernel<EPI_SWIGLU>, dim3(2 * pairs), dim3(THREADS), smem_bytes_of(EPI_SWIGLU), stream, 2,
                             tm_a, tm_b, tm_h, A_s, B_s, H, H_s, M, I, K, tiles, 0, 1, K / BK, no_partials, no_counters,
                             GatherDst{}, RopeHook{}, info->status));
   g_launches.fetch_add(1);
@@ -1328,13 +1364,13 @@ static int launch_fp8_gather(const void*       A,
   static thread_local bool attr_set[64] = {};
   if (!attr_set[info->device]) {
     LLMMM_CUDA_TRY(cudaFuncSetAttribute(
-      fp8_blockwise_gemm_pair_kernel<EPI_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES_STAGED));
+      fp8_blockwise_gemm_pair_kernel<EPI_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes_of(EPI_GATHER)));
     attr_set[info->device] = true;
   }
   const int       tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   const SplitPlan plan  = plan_split(info, tiles, K / BK, /*fixed*/ 4, /*per_way_x2*/ 5, /*min_gain*/ 3);
   float*          none  = nullptr;
-  LLMMM_CUDA_TRY(launch_pdl(fp8_blockwise_gemm_pair_kernel<EPI_GATHER>, dim3(2 * plan.pairs), dim3(THREADS), SMEM_BYTES_STAGED, stream, 2,
+  LLMMM_CUDA_TRY(launch_pdl(fp8_blockwise_gemm_pair_kernel<EPI_GATHER>, dim3(2 * plan.pairs), dim3(THREADS), smem_bytes_of(EPI_GATHER), stream, 2,
                             tm_a, tm_b, CUtensorMap{}, A_s, B_s, static_cast<void*>(nullptr), none, M, N, K, plan.dp_tiles, plan.split_pairs,
                             plan.split_s, plan.split_chunk, plan.partials, plan.counters, dst, RopeHook{}, info->status));
   g_launches.fetch_add(1);
@@ -1427,11 +1463,11 @@ int launch_fp8_e4m3(const void* A, const float* A_s, const void* B, const float*
 int warm_fp8_kernels(const DeviceInfo* info)
 {
   (void)info;
-  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_E4M3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::SMEM_BYTES_STAGED));
-  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::SMEM_BYTES_STAGED));
-  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::SMEM_BYTES_SWIGLU));
-  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::SMEM_BYTES_STAGED));
-  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::SMEM_BYTES_ROPE));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_E4M3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_E4M3)));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_F32)));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_SWIGLU)));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_GATHER)));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_ROPE)));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8cfg::SMEM_BYTES));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8cfg::SMEM_BYTES));
   return warm_decode_kernels(info);

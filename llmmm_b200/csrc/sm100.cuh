@@ -150,6 +150,53 @@ mbar_wait(uint64_t* bar, uint32_t parity, uint32_t code, volatile uint32_t* abor
   mbar_wait_limit(bar, parity, code, abort_flag, status, WAIT_LIMIT_NS);
 }
 
+// The same with the barrier and the abort flag given as shared-memory addresses (half the registers of pointers).
+__device__ __forceinline__ void mbar_arrive_at(uint32_t bar_addr)
+{
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_addr) : "memory");
+}
+
+__device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar_addr, uint32_t parity)
+{
+  uint32_t ok;
+  asm volatile("{\n\t"
+               ".reg .pred p;\n\t"
+               "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+               "selp.u32 %0, 1, 0, p;\n\t"
+               "}"
+               : "=r"(ok)
+               : "r"(bar_addr), "r"(parity)
+               : "memory");
+  return ok != 0;
+}
+
+__device__ __forceinline__ void mbar_wait_at(uint32_t bar_addr, uint32_t parity, uint32_t code, uint32_t abort_addr, uint32_t* status)
+{
+  if (mbar_try_wait_at(bar_addr, parity)) {
+    return;
+  }
+  unsigned long long t0    = 0;
+  uint32_t           spins = 0;
+  while (!mbar_try_wait_at(bar_addr, parity)) {
+    if ((++spins & 0x3ff) == 0) {
+      uint32_t aborted;
+      asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(aborted) : "r"(abort_addr) : "memory");
+      if (aborted) {
+        return;
+      }
+      const unsigned long long now = global_timer_ns();
+      if (t0 == 0) {
+        t0 = now;
+      }
+      else if (now - t0 > WAIT_LIMIT_NS) {
+        asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_addr), "r"(code) : "memory");
+        atomicCAS(status, 0u, code);
+        return;
+      }
+    }
+  }
+}
+
 // ------------------------------------------- programmatic dependent launch ---
 //
 // A kernel launched with cudaLaunchAttributeProgrammaticStreamSerialization may start while its

@@ -82,6 +82,15 @@ def test_general_kernel_small_shapes(capi, oracle, cuda, shape):
     check_against_oracle(oracle, *case, gq, gs, gf)
 
 
+@pytest.mark.parametrize("k_blocks", [1, 3, 4, 5, 17, 21])
+@pytest.mark.parametrize("M", [129, 254, 387])
+def test_pair_kernel_scale_ring(capi, oracle, cuda, M, k_blocks):
+    # K-blocks around the chunks of four and the sixteen of the whole ring in which the pair kernel keeps its scales;
+    # an odd number of rows, so that rows of A_s start at any multiple of four bytes; several tiles per pair
+    case = make_case(oracle, 46 + k_blocks, M, 384, 128 * k_blocks)
+    check_against_oracle(oracle, *case, *gpu_mm(capi, cuda, *case))
+
+
 @pytest.mark.parametrize("M", [1, 2, 15, 16, 17, 33, 64])
 @pytest.mark.parametrize("NK", [(256, 1024), (384, 128), (2560, 4096), (19072, 256), (37888, 128), (25600, 512)])
 def test_decode_kernel_ragged_m(capi, oracle, cuda, M, NK):
