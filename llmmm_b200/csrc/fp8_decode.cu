@@ -1116,6 +1116,18 @@ size_t decode_workspace_bytes(int M)
   return split_workspace_bytes() + decode_partial_bytes(M);
 }
 
+size_t decode_acc_offset(int M, int cols)
+{
+  const size_t acc = (size_t)M * cols * sizeof(float);
+  return WS_HEADER_BYTES + acc <= split_workspace_bytes() ? WS_HEADER_BYTES : (decode_workspace_bytes(64) + 255) & ~size_t(255);
+}
+
+size_t decode_acc_workspace_bytes(int M, int cols)
+{
+  const size_t end = decode_acc_offset(M, cols) + (size_t)M * cols * sizeof(float);
+  return end > decode_workspace_bytes(M) ? end : decode_workspace_bytes(M);
+}
+
 namespace {
 thread_local Workspace t_ws;
 thread_local bool      t_ws_bound = false;

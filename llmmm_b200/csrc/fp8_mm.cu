@@ -1670,12 +1670,11 @@ int llmmm_fp8_blockwise_mm_swiglu_e4m3out(const void*    A,
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (M <= 64) {
     // Decode-sized: the weight-streaming decode kernel leaves the [M, 2I] accumulator in the registered scratch
-    // (behind its own partial tiles) and a second, tiny kernel applies SwiGLU and quantises.  Without enough
+    // (decode_acc_offset) and a second, tiny kernel applies SwiGLU and quantises.  Without enough
     // scratch the 256-row kernel below runs (correct, but it reads the weights at a fraction of the rate).
-    const Workspace ws  = registered_workspace(info->device);
-    const size_t    off = (decode_workspace_bytes(M) + 255) & ~size_t(255);
-    if (ws.ptr != nullptr && ws.bytes >= off + (size_t)M * 2 * I * sizeof(float)) {
-      float*    acc = reinterpret_cast<float*>(static_cast<uint8_t*>(ws.ptr) + off);
+    const Workspace ws = registered_workspace(info->device);
+    if (ws.ptr != nullptr && ws.bytes >= decode_acc_workspace_bytes(M, 2 * I)) {
+      float*    acc = reinterpret_cast<float*>(static_cast<uint8_t*>(ws.ptr) + decode_acc_offset(M, 2 * I));
       const int rc  = launch_decode(true, A, A_scale_t, B_gate_up_t, B_scale_t, acc, nullptr, M, 2 * I, K, s);
       if (rc == LLMMM_OK) {
         return launch_swiglu_quant(acc, H, H_scale_t, M, I, s);
@@ -1742,12 +1741,11 @@ int llmmm_fp8_blockwise_mm_qk_norm_rope_e4m3out(const void*    A,
   cudaStream_t   s = reinterpret_cast<cudaStream_t>(stream);
   if (M <= 64) {
     // Decode-sized: the weight-streaming decode kernel leaves the [M, N] accumulator in the registered scratch
-    // (behind its own partial tiles) and a second, tiny kernel applies the hook and quantises.  Without enough
+    // (decode_acc_offset) and a second, tiny kernel applies the hook and quantises.  Without enough
     // scratch the 256-row kernel below runs (correct, but it reads the weights at a fraction of the rate).
-    const Workspace ws  = registered_workspace(info->device);
-    const size_t    off = (decode_workspace_bytes(M) + 255) & ~size_t(255);
-    if (ws.ptr != nullptr && ws.bytes >= off + (size_t)M * N * sizeof(float)) {
-      float*    acc = reinterpret_cast<float*>(static_cast<uint8_t*>(ws.ptr) + off);
+    const Workspace ws = registered_workspace(info->device);
+    if (ws.ptr != nullptr && ws.bytes >= decode_acc_workspace_bytes(M, N)) {
+      float*    acc = reinterpret_cast<float*>(static_cast<uint8_t*>(ws.ptr) + decode_acc_offset(M, N));
       const int rc  = launch_decode(true, A, A_scale_t, B_t, B_scale_t, acc, nullptr, M, N, K, s);
       if (rc == LLMMM_OK) {
         return launch_rope_quant(acc, C, C_scale_t, hook, M, N, info->status, s);
@@ -1772,7 +1770,7 @@ size_t llmmm_fp8_qk_norm_rope_workspace_bytes(int M, int N, int K)
   if (M > 64) {
     return 0;  // the fused kernel runs whole tiles and needs no scratch
   }
-  return ((llmmm::decode_workspace_bytes(M) + 255) & ~size_t(255)) + (size_t)M * N * sizeof(float);
+  return llmmm::decode_acc_workspace_bytes(M, N);
 }
 
 size_t llmmm_fp8_swiglu_workspace_bytes(int M, int I, int K)
@@ -1781,7 +1779,7 @@ size_t llmmm_fp8_swiglu_workspace_bytes(int M, int I, int K)
   if (M < 1 || M > 64 || I < 128) {
     return 0;  // larger M: the fused kernel needs no scratch
   }
-  return ((llmmm::decode_workspace_bytes(M) + 255) & ~size_t(255)) + (size_t)M * 2 * I * sizeof(float);
+  return llmmm::decode_acc_workspace_bytes(M, 2 * I);
 }
 
 int llmmm_fp8_blockwise_mm_f32out(const void*    A,

@@ -118,6 +118,12 @@ int check_workspace_arg(const void* ptr, size_t bytes);
 size_t split_workspace_bytes();
 // Scratch of the decode kernel for M rows (header + partial tiles), fp8_decode.cu.
 size_t decode_workspace_bytes(int M);
+// Where the decode-sized forms of the hooks (SwiGLU, q/k norm + RoPE) leave their fp32 accumulator [M, cols] in the
+// scratch, and how much scratch that takes: in the pair kernels' partial tiles, which a decode-sized call does not
+// use and which hold anything between launches; a larger one behind the decode kernel's words for ANY M.  (Behind
+// the words for this M it would lie inside those of a call with more rows, which must be zero between launches.)
+size_t decode_acc_offset(int M, int cols);
+size_t decode_acc_workspace_bytes(int M, int cols);
 // SwiGLU + 1x128 quantisation of a gate_up accumulator acc [M, 2I] fp32 (quant.cu): the second step of the
 // decode-sized form of llmmm_fp8_blockwise_mm_swiglu_e4m3out.
 int launch_swiglu_quant(const float* acc, void* H, float* H_s, int M, int I, cudaStream_t stream);

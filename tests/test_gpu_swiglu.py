@@ -129,6 +129,28 @@ def test_swiglu_decode_sized(capi, oracle, cuda, M, IK):
     assert np.array_equal(gq2, gq3) and np.array_equal(gs2.view(np.uint32), gs3.view(np.uint32))
 
 
+@pytest.mark.parametrize("M", [33, 64])
+def test_decode_call_after_a_hook_call_with_fewer_rows(capi, oracle, cuda, M):
+    # The hook's accumulator stays in the scratch.  It must not lie where a later call with more rows keeps the words
+    # of its cut output groups, which have to be zero between launches.
+    I, K = 9728, 2560  # 152 output groups on 148 SMs: four of them are cut among 80 CTAs
+    I_hook = 28672     # large enough for its accumulator to cover the words of a whole cut group
+    capi.clear_workspace()
+    capi.ensure_swiglu_workspace(16, I_hook, 256)
+    capi.ensure_workspace(M, 2 * I, K)
+    case = make_case(oracle, 97, M, I, K)
+    dA, dAs, dB, dBs = to_dev(cuda, *case)
+    outs = []
+    for hook_first in (False, True):
+        if hook_first:
+            run(capi, cuda, make_case(oracle, 98, 16, I_hook, 256), 16, I_hook, 256, launches=2)
+        C = torch.full((M, 2 * I), float("nan"), device=cuda)
+        capi.fp8_blockwise_mm_f32(dA, dAs, dB, dBs, C, M, 2 * I, K)
+        torch.cuda.synchronize()
+        outs.append(C)
+    assert torch.equal(*outs)
+
+
 def test_swiglu_argument_errors(capi, cuda):
     z8 = torch.zeros(256, 256, dtype=torch.uint8, device=cuda)
     zf = torch.zeros(256, 256, device=cuda)
