@@ -1,4 +1,4 @@
-"""Builds libllmmm_b200.so (the C-ABI library) in-tree with nvcc for sm_100a.
+"""Builds libllmmm_b200.so (the C-ABI library) in-tree with nvcc for sm_100a, and _binding.so (its calls for Python).
 
 Usage: python -m llmmm_b200.build [--force] [--verbose] [--profile]
 
@@ -13,12 +13,14 @@ import concurrent.futures as cf
 import os
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "libllmmm_b200.so"
+BINDING = PKG / "_binding.so"
 PROFILE_LIB = PKG / "libllmmm_b200_profile.so"
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
@@ -87,7 +89,26 @@ def build_library(force: bool = False, verbose: bool = False, profile: bool = Fa
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    if not profile:
+        build_binding(force)
     return lib
+
+
+def build_binding(force: bool = False) -> Path:
+    """_binding.so: the native form of the calls in capi.py, against the headers of the torch it will run with."""
+    src = CSRC / "binding.cpp"
+    if not force and _newer(BINDING, [src, PKG.parent / "include" / "llmmm_c.h"]):
+        return BINDING
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{root / 'include'}", f"-I{root / 'include/torch/csrc/api/include'}", f"-I{Path(NVCC).resolve().parent.parent / 'include'}",
+           f"-I{sysconfig.get_paths()['include']}", str(src), "-o", str(BINDING), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch",
+           "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-L{PKG}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{src.name}: {r.stdout}\n{r.stderr}")
+    return BINDING
 
 
 if __name__ == "__main__":

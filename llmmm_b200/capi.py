@@ -8,6 +8,10 @@ Python counterpart of the reference's std::runtime_error.
 
 torch is used only to hold device memory and to name the current stream.
 There is no fallback: if the shared library is missing, loading raises.
+
+The calls a token loop makes go through `_binding` (csrc/binding.cpp), which
+makes the same call of the same library in a fifth of the host time; what it
+does not take (it returns False) goes through ctypes below.
 """
 from __future__ import annotations
 
@@ -15,6 +19,11 @@ import ctypes
 from pathlib import Path
 
 import torch
+
+try:
+    from . import _binding as _native
+except ImportError:  # built against another torch, or not built: ctypes only
+    _native = None
 
 _LIB_PATH = Path(__file__).resolve().parent / "libllmmm_b200.so"
 _lib = None
@@ -115,6 +124,8 @@ def check_status(stream=None) -> None:
 
 def fp16_mm(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor, M: int, N: int, K: int, stream=None) -> None:
     """C[M,N] = A[M,K] @ B[K,N] for half / bfloat16 (LLMMM::fp16_mm<T>)."""
+    if _native is not None and _native.fp16_mm(A, B, C, M, N, K, stream):
+        return
     if A.dtype == torch.float16:
         fn = lib().llmmm_fp16_mm_f16
     elif A.dtype == torch.bfloat16:
@@ -128,6 +139,8 @@ def fp16_mm(A: torch.Tensor, B: torch.Tensor, C: torch.Tensor, M: int, N: int, K
 def fp8_blockwise_mm(A_q, A_s, B_q, B_s, C_q, C_s, M: int, N: int, K: int, stream=None) -> None:
     """FP8 blockwise GEMM, e4m3 output with fused 1x128 scales
     (fp8_gemm_blockwise_quant_A_1x128__B_128x128__C_1x128__output_fp8*)."""
+    if _native is not None and _native.fp8_blockwise_mm(A_q, A_s, B_q, B_s, C_q, C_s, M, N, K, stream):
+        return
     with torch.cuda.device(A_q.device):
         _check(lib().llmmm_fp8_blockwise_mm_e4m3out(
             _dev(A_q), _dev(A_s, torch.float32), _dev(B_q), _dev(B_s, torch.float32), _dev(C_q),
@@ -198,6 +211,8 @@ def fp8_blockwise_mm_gather(A_q, A_s, B_q, B_s, C_dsts, Cs_dsts, N_total: int, c
 def fp8_blockwise_mm_swiglu(A_q, A_s, B_gate_up_q, B_s, H_q, H_s, M: int, I: int, K: int, stream=None) -> None:
     """gate_up projection [2I, K] with the SwiGLU epilogue fused: H = silu(gate) * up, quantised 1x128 along I
     into H_q [M, I] / H_s [I/128, M] (the A operand of the down projection)."""
+    if _native is not None and _native.fp8_blockwise_mm_swiglu(A_q, A_s, B_gate_up_q, B_s, H_q, H_s, M, I, K, stream):
+        return
     with torch.cuda.device(A_q.device):
         _check(lib().llmmm_fp8_blockwise_mm_swiglu_e4m3out(
             _dev(A_q), _dev(A_s, torch.float32), _dev(B_gate_up_q), _dev(B_s, torch.float32), _dev(H_q),
@@ -212,6 +227,9 @@ def fp8_blockwise_mm_qk_norm_rope(A_q, A_s, B_q, B_s, C_q, C_s, positions, cos, 
     by check_status()."""
     if cos.shape != sin.shape or cos.dim() != 2 or cos.shape[1] != 64:
         raise RuntimeError("cos and sin must both be [rows, 64]")
+    if _native is not None and _native.fp8_blockwise_mm_qk_norm_rope(A_q, A_s, B_q, B_s, C_q, C_s, positions, cos, sin, q_weight, k_weight, eps,
+                                                                     n_q_heads, n_kv_heads, M, N, K, stream):
+        return
     with torch.cuda.device(A_q.device):
         _check(lib().llmmm_fp8_blockwise_mm_qk_norm_rope_e4m3out(
             _dev(A_q), _dev(A_s, torch.float32), _dev(B_q), _dev(B_s, torch.float32), _dev(C_q),
@@ -230,6 +248,8 @@ def ensure_qk_norm_rope_workspace(M: int, N: int, K: int, device=None) -> None:
 def fp8_blockwise_mm_f32(A_q, A_s, B_q, B_s, C, M: int, N: int, K: int, stream=None) -> None:
     """FP8 blockwise GEMM, fp32 output
     (fp8_gemm_blockwise_quant_A_1x128__B_128x128__output_fp32)."""
+    if _native is not None and _native.fp8_blockwise_mm_f32(A_q, A_s, B_q, B_s, C, M, N, K, stream):
+        return
     with torch.cuda.device(A_q.device):
         _check(lib().llmmm_fp8_blockwise_mm_f32out(
             _dev(A_q), _dev(A_s, torch.float32), _dev(B_q), _dev(B_s, torch.float32), _dev(C, torch.float32),
@@ -238,6 +258,8 @@ def fp8_blockwise_mm_f32(A_q, A_s, B_q, B_s, C, M: int, N: int, K: int, stream=N
 
 def fp8_quant_1x128(x, q, scale, M: int, K: int, stream=None) -> None:
     """fp8_blockwise_symmetric_quantization<1,128,true>."""
+    if _native is not None and _native.fp8_quant_1x128(x, q, scale, M, K, stream):
+        return
     with torch.cuda.device(x.device):
         _check(lib().llmmm_fp8_quant_1x128(_dev(x, torch.float32), _dev(q), _dev(scale, torch.float32), M, K,
                                            _stream(stream)))
@@ -245,6 +267,8 @@ def fp8_quant_1x128(x, q, scale, M: int, K: int, stream=None) -> None:
 
 def fp8_rmsnorm_quant_1x128(x, weight, eps: float, q, scale, M: int, K: int, stream=None) -> None:
     """y = x * rsqrt(mean(x^2) + eps) * weight per row, then the 1x128 quantisation of y (one kernel)."""
+    if _native is not None and _native.fp8_rmsnorm_quant_1x128(x, weight, eps, q, scale, M, K, stream):
+        return
     with torch.cuda.device(x.device):
         _check(lib().llmmm_fp8_rmsnorm_quant_1x128(_dev(x, torch.float32), _dev(weight, torch.float32), ctypes.c_float(eps),
                                                    _dev(q), _dev(scale, torch.float32), M, K, _stream(stream)))
@@ -252,6 +276,8 @@ def fp8_rmsnorm_quant_1x128(x, weight, eps: float, q, scale, M: int, K: int, str
 
 def fp8_quant_128x128(x, q, scale, rows: int, cols: int, stream=None) -> None:
     """fp8_blockwise_symmetric_quantization<128,128,false>."""
+    if _native is not None and _native.fp8_quant_128x128(x, q, scale, rows, cols, stream):
+        return
     with torch.cuda.device(x.device):
         _check(lib().llmmm_fp8_quant_128x128(_dev(x, torch.float32), _dev(q), _dev(scale, torch.float32), rows,
                                              cols, _stream(stream)))
