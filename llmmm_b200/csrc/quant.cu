@@ -16,13 +16,12 @@
 
 namespace llmmm {
 
+// Largest of the warp's values, all of them non-negative or NaN: one integer reduction (the bit patterns of
+// non-negative floats order like the floats; five shuffles and maxima were the longest chain of these kernels).  Like
+// fmaxf it passes NaN over unless every value is one.
 __device__ __forceinline__ float warp_max(float v)
 {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  }
-  return v;
+  return __int_as_float(__reduce_max_sync(0xffffffffu, v == v ? __float_as_int(v) : -1));
 }
 
 __device__ __forceinline__ float amax4(float4 v)
@@ -67,9 +66,9 @@ __device__ __forceinline__ uint32_t quant4(float4 v, float s)
 // the 32 lanes hold one float4 each (a coalesced 512-byte read, all rows' loads in
 // flight together), the row amax is a warp reduction, and lane r keeps the scale
 // of row r so that the scales leave as one 32-byte sector of scale[(K/128), M].
-constexpr int Q1_ROWS  = 8;
 constexpr int Q1_WARPS = 8;
 
+template<int Q1_ROWS>
 __global__ void __launch_bounds__(Q1_WARPS * 32)
   quant_1x128_kernel(const float* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale, int M, int K)
 {
@@ -87,29 +86,23 @@ __global__ void __launch_bounds__(Q1_WARPS * 32)
   const int g  = (int)(w % groups);
   const int m0 = (int)(w / groups) * Q1_ROWS;
 
-  float my_scale = 0.0f;
-#pragma unroll 1
-  for (int r0 = 0; r0 < Q1_ROWS; r0 += 8) {
-    float4 v[8];
+  float  my_scale = 0.0f;
+  float4 v[Q1_ROWS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int m = m0 + r0 + j;
-      v[j]        = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (m < M) {
-        v[j] = __ldcs(reinterpret_cast<const float4*>(x + (size_t)m * K + (size_t)g * 128) + lane);
-      }
+  for (int j = 0; j < Q1_ROWS; ++j) {
+    const int m = m0 + j;
+    v[j]        = m < M ? __ldcs(reinterpret_cast<const float4*>(x + (size_t)m * K + (size_t)g * 128) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int j = 0; j < Q1_ROWS; ++j) {
+    const int   m    = m0 + j;
+    const float amax = warp_max(amax4(v[j]));
+    const float s    = __fdiv_rn(amax, 448.0f);
+    if (lane == j) {
+      my_scale = s;
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int   m    = m0 + r0 + j;
-      const float amax = warp_max(amax4(v[j]));
-      const float s    = __fdiv_rn(amax, 448.0f);
-      if (lane == r0 + j) {
-        my_scale = s;
-      }
-      if (m < M) {
-        reinterpret_cast<uint32_t*>(q + (size_t)m * K + (size_t)g * 128)[lane] = quant4(v[j], s);
-      }
+    if (m < M) {
+      reinterpret_cast<uint32_t*>(q + (size_t)m * K + (size_t)g * 128)[lane] = quant4(v[j], s);
     }
   }
   if (lane < Q1_ROWS && m0 + lane < M) {
@@ -164,10 +157,9 @@ __global__ void __launch_bounds__(256)
 // quantisation of y.  One CTA per row: it sums the squares, then scales and quantises one 128-wide group per
 // warp at a time.  A row of up to 8192 values is kept in registers in between (one pass over memory); a longer
 // one is re-read from L2.
-constexpr int RN_THREADS = 256;
 
 // RESIDENT: float4 values of the row a thread keeps (0: none, the row is re-read from L2 for the second phase).
-template<int RESIDENT>
+template<int RN_THREADS, int RESIDENT>
 __global__ void __launch_bounds__(RN_THREADS)
   rmsnorm_quant_1x128_kernel(const float* __restrict__ x, const float* __restrict__ weight, float eps, uint8_t* __restrict__ q,
                              float* __restrict__ scale, int M, int K)
@@ -179,8 +171,8 @@ __global__ void __launch_bounds__(RN_THREADS)
   const int     warp = threadIdx.x >> 5;
   const int     m    = blockIdx.x;
   const float4* row  = reinterpret_cast<const float4*>(x + (size_t)m * K);
-  // Rows of up to 8192 values stay in registers between the two phases (RESIDENT float4 per thread): element
-  // threadIdx.x + 256 j of the row, as float4, is lane `lane` of the 128-wide group warp + 8 j, so the thread
+  // The row stays in registers between the two phases (RESIDENT float4 per thread): element threadIdx.x +
+  // RN_THREADS j of the row, as float4, is lane `lane` of the 128-wide group warp + RN_THREADS / 32 j, so the thread
   // that read a value for the sum of squares is the one that quantises it, and x is read from memory once.
   constexpr bool resident = RESIDENT > 0;
   float4         v[resident ? RESIDENT : 1];
@@ -390,15 +382,28 @@ int llmmm_fp8_rmsnorm_quant_1x128(const float* x, const float* weight, float eps
   if (!(eps >= 0.0f)) {
     return set_error(LLMMM_ERR_SHAPE, "eps must be non-negative");
   }
-  if (device_info() == nullptr) {
+  const DeviceInfo* device = device_info();
+  if (device == nullptr) {
     return LLMMM_ERR_UNSUPPORTED;
   }
-  // as few resident values as the row needs: registers decide how many rows an SM works on at a time
-  auto* kernel = K <= 2 * RN_THREADS * 4 ? rmsnorm_quant_1x128_kernel<2>
-               : K <= 4 * RN_THREADS * 4 ? rmsnorm_quant_1x128_kernel<4>
-               : K <= 8 * RN_THREADS * 4 ? rmsnorm_quant_1x128_kernel<8> : rmsnorm_quant_1x128_kernel<0>;
-  LLMMM_CUDA_TRY(launch_pdl(kernel, dim3((unsigned)M), dim3(RN_THREADS), 0,
-                            reinterpret_cast<cudaStream_t>(stream), 1, x, weight, eps, static_cast<uint8_t*>(q), scale, M, K));
+  auto launch = [&](auto* kernel, int threads) {
+    return launch_pdl(kernel, dim3((unsigned)M), dim3((unsigned)threads), 0, reinterpret_cast<cudaStream_t>(stream), 1, x, weight, eps,
+                      static_cast<uint8_t*>(q), scale, M, K);
+  };
+  // Up to a row per SM a row is a latency: as many threads as share it well (M = 1, K = 2560: 512 threads 2.3 us, 256 2.6, 128
+  // 3.2).  More rows: as few resident values as the row needs, registers decide how many rows an SM works on at a time;
+  // short rows in large numbers run best with more, smaller CTAs (4096 x 2560: 128 threads 13.4 us, 256 14.6; 1333 x 2560:
+  // 5.9 and 5.4; 8192 x 3584: 30.2 and 31.5 us).
+  const bool few = M <= device->sm_count;
+  LLMMM_CUDA_TRY(K > 8192        ? launch(rmsnorm_quant_1x128_kernel<256, 0>, 256)
+                 : few && K > 4096 ? launch(rmsnorm_quant_1x128_kernel<512, 4>, 512)
+                 : few && K > 2048 ? launch(rmsnorm_quant_1x128_kernel<512, 2>, 512)
+                 : few             ? launch(rmsnorm_quant_1x128_kernel<512, 1>, 512)
+                 : K > 4096        ? launch(rmsnorm_quant_1x128_kernel<256, 8>, 256)
+                 : K > 3072        ? launch(rmsnorm_quant_1x128_kernel<256, 4>, 256)
+                 : K > 2048 && K <= 2560 && M >= 2048 ? launch(rmsnorm_quant_1x128_kernel<128, 5>, 128)
+                 : K > 2048        ? launch(rmsnorm_quant_1x128_kernel<256, 3>, 256)
+                                   : launch(rmsnorm_quant_1x128_kernel<256, 2>, 256));
   g_launches.fetch_add(1);
   return LLMMM_OK;
 }
@@ -418,10 +423,20 @@ int llmmm_fp8_quant_1x128(const float* x, void* q, float* scale, int M, int K, l
   if (device_info() == nullptr) {
     return LLMMM_ERR_UNSUPPORTED;
   }
-  const long long warps  = (long long)((M + Q1_ROWS - 1) / Q1_ROWS) * (K / 128);
-  const long long blocks = (warps + Q1_WARPS - 1) / Q1_WARPS;
-  LLMMM_CUDA_TRY(launch_pdl(quant_1x128_kernel, dim3((unsigned)blocks), dim3(Q1_WARPS * 32), 0,
-                            reinterpret_cast<cudaStream_t>(stream), 1, x, static_cast<uint8_t*>(q), scale, M, K));
+  auto launch = [&](auto* kernel, int rows) {
+    const long long warps  = (long long)((M + rows - 1) / rows) * (K / 128);
+    const long long blocks = (warps + Q1_WARPS - 1) / Q1_WARPS;
+    return launch_pdl(kernel, dim3((unsigned)blocks), dim3(Q1_WARPS * 32), 0, reinterpret_cast<cudaStream_t>(stream), 1, x,
+                      static_cast<uint8_t*>(q), scale, M, K);
+  };
+  // Rows per warp: one while the groups are few (a warp's chain is what the call takes: 1 x 4096 1.5 us against 2.9 us with
+  // eight), more rows amortise a warp's start and fill its sector of the scales (8192 x 3584: one 38.0, two 30.2, four
+  // 26.2, eight 25.5 us; 1333 x 2560: 5.6, 4.7, 4.7, 5.0 us).
+  const long long groups = (long long)M * (K / 128);
+  LLMMM_CUDA_TRY(groups <= 4096     ? launch(quant_1x128_kernel<1>, 1)
+                 : groups <= 16384  ? launch(quant_1x128_kernel<2>, 2)
+                 : groups <= 131072 ? launch(quant_1x128_kernel<4>, 4)
+                                    : launch(quant_1x128_kernel<8>, 8));
   g_launches.fetch_add(1);
   return LLMMM_OK;
 }

@@ -50,6 +50,39 @@ def test_quant_128x128_bit_exact(capi, oracle, cuda, shape):
     assert (q == oq).all()
 
 
+@pytest.mark.parametrize("shape", [(4096, 128), (4097, 128), (5461, 384), (5462, 384), (7711, 2176), (7710, 2176)])
+def test_quant_1x128_rows_per_warp(capi, cuda, shape):
+    # both sides of the group counts (4096, 16384, 131072) at which a warp takes more rows, against torch's IEEE divisions
+    M, K = shape
+    x = torch.randn(M, K, device=cuda, generator=torch.Generator(device=cuda).manual_seed(33))
+    x[M // 2] *= 1e20
+    q = torch.full((M, K), 0xAA, dtype=torch.uint8, device=cuda)
+    s = torch.full((K // 128, M), float("nan"), device=cuda)
+    capi.fp8_quant_1x128(x, q, s, M, K)
+    b = x.view(M, K // 128, 128)
+    want = b.abs().amax(dim=2) / torch.full((), 448.0, device=cuda)
+    assert torch.equal(s.t(), want)
+    assert torch.equal(q, (b / want[..., None]).to(torch.float8_e4m3fn).view(torch.uint8).view(M, K))
+
+
+def test_quant_1x128_nan_and_infinity(capi, cuda):
+    # NaN values do not enter a group's maximum unless all of them are NaN; an infinite value makes the scale infinite
+    x = torch.randn(3, 256, device=cuda, generator=torch.Generator(device=cuda).manual_seed(34))
+    clean = x.clone()
+    x[0, 5], x[0, 6] = float("nan"), -float("nan")
+    x[1, :128] = float("nan")
+    x[2, 130] = float("-inf")
+    q = torch.zeros(3, 256, dtype=torch.uint8, device=cuda)
+    s = torch.zeros(2, 3, device=cuda)
+    capi.fp8_quant_1x128(x, q, s, 3, 256)
+    rest = clean.clone()
+    rest[0, 5:7] = 0
+    assert s[0, 0] == rest[0, :128].abs().max() / torch.full((), 448.0, device=cuda)
+    assert bool(((q[0, 5:7] & 0x7F) == 0x7F).all()) and bool(((q[0, 7:128] & 0x7F) != 0x7F).all())
+    assert bool(torch.isnan(s[0, 1])) and bool(((q[1, :128] & 0x7F) == 0x7F).all())
+    assert bool(torch.isinf(s[1, 2])) and bool(torch.isfinite(s[1, :2]).all())
+
+
 def test_full_size_quant_properties(capi, cuda):
     # 4096 x 4096 (the FP8 headline config): every group's largest code is +-448 and the
     # scale array is exactly amax/448 computed by torch in fp32

@@ -27,7 +27,11 @@ def run(capi, cuda, x, w, eps):
     return q.cpu().numpy(), s.cpu().numpy()
 
 
-@pytest.mark.parametrize("shape", [(1, 128), (16, 2560), (33, 384), (64, 9728), (257, 1024), (512, 18944)])
+@pytest.mark.parametrize("shape", [(1, 128), (16, 2560), (33, 384), (64, 9728), (257, 1024), (512, 18944),
+                                   # the edges between the instantiations: K 2048, 2560, 3072, 4096, 8192, a row per SM, 2048 rows
+                                   (3, 2048), (3, 2176), (3, 4096), (3, 4224), (3, 8192), (3, 8320), (148, 2048), (149, 2048), (149, 2176),
+                                   (149, 3072), (149, 3200), (149, 4096), (149, 4224), (149, 8192), (149, 8320), (2047, 2560), (2048, 2560),
+                                   (2048, 2688)])
 def test_rmsnorm_quant_against_oracle(capi, oracle, cuda, shape):
     M, K = shape
     rng = np.random.default_rng(100 + M)
