@@ -131,6 +131,7 @@ struct DecodeBars {
   uint64_t red;  // cluster kernel: the other CTAs' partials of this CTA's rows have landed (counted in bytes)
   float    amax[4][64];
   float    inv[64];
+  float    row_max[2][4];  // reduction warps
 };
 static_assert(sizeof(DecodeBars) <= 1536, "DecodeBars outgrew its slot in shared memory");
 
@@ -230,18 +231,18 @@ __device__ __forceinline__ void store_group_row(float4 s, int m, int nb, void* _
   }
 }
 
-// Cheap wait in front of the reduction of a split group: lane j polls ONE word of contributor j's partial tile (in
-// the first row this warp owns: nobody else puts that word back to zero), so that a warp that is early does not
+// Cheap wait in front of the reduction of a split group: lane j polls ONE word of contributor j's partial tile (one
+// that only this warp puts back to zero), so that a warp that is early does not
 // keep re-reading whole rows of every contributor -- hundreds of warps doing that would load the L2 with
 // megabytes per polling round.  Only a hint: stores may land in any order, and the reduction still checks
 // every word it uses.  Bounded like every wait.
 template<int MP>
-__device__ __forceinline__ bool wait_contributors(const SplitGroup& g, const uint32_t* partials, int lane,
+__device__ __forceinline__ bool wait_contributors(const SplitGroup& g, const uint32_t* partials, int row, int column, int lane,
                                                   volatile uint32_t* abort_flag, uint32_t* status)
 {
   for (int base = 0; base < g.cnt; base += 32) {
     const int          j     = base + lane;
-    const uint32_t*    word  = partials + ((size_t)((g.c_lo + j) * 2 + (j == 0 ? 1 : 0)) * MP + g.gw) * 128 + 127;
+    const uint32_t*    word  = partials + ((size_t)((g.c_lo + j) * 2 + (j == 0 ? 1 : 0)) * MP + row) * 128 + column;
     unsigned long long t0    = 0;
     uint32_t           spins = 0;
     for (;;) {
@@ -426,6 +427,85 @@ __device__ __forceinline__ bool reduce_split_groups(const SplitGroup (&g)[NG],
   return true;
 }
 
+// The same for ONE group with many contributors (a left-over group of a shape with at least as many groups as CTAs is cut
+// into pieces of one or two K-blocks) and few rows: contributor j's four reduction warps take rows j, j + cnt, ...
+// together, 32 columns each, one word per lane and contributor, so that CB contributors are in flight in CB registers.
+// With a warp per row (four words per lane, eight contributors in flight) the rows were finished two loaded L2 round
+// trips later, and the launch with them (19456x2560 at M = 1 / 16: 11.6 / 12.2 us, now 10.6 / 11.1 us).
+template<int MP, bool OUT_F32, int CB>
+__device__ __forceinline__ void reduce_split_group_rows(const SplitGroup& g, int j0, int rw, float (&row_max)[2][4],
+                                                        uint32_t* __restrict__ partials, void* __restrict__ C_out, float* __restrict__ C_s,
+                                                        int M, int N, int lane, volatile uint32_t* abort_flag, uint32_t* status)
+{
+  const int n = rw * 32 + lane;  // column inside the group
+  for (int m = j0, turn = 0; m < M; m += g.cnt, turn ^= 1) {
+    float sum = 0.0f;
+    for (int base = 0; base < g.cnt; base += CB) {
+      uint32_t*          src = partials + ((size_t)((g.c_lo + base) * 2) * MP + m) * 128 + n;
+      uint32_t           w[CB];
+      unsigned long long t0    = 0;
+      uint32_t           spins = 0;
+      for (;;) {
+        bool landed = true;
+#pragma unroll
+        for (int j = 0; j < CB; ++j) {
+          w[j] = 1u;
+          if (base + j < g.cnt) {
+            // (the group's first contributor reached it at K-block 0: slot 1)
+            asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(w[j]) : "l"(src + (j * 2 + (base + j == 0 ? 1 : 0)) * (MP * 128)) : "memory");
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < CB; ++j) {
+          landed = landed && w[j] != 0u;
+        }
+        if (__all_sync(0xffffffffu, landed)) {
+          break;
+        }
+        if ((++spins & 0x7) == 0) {
+          if (*abort_flag) {
+            break;  // (not a return: the four warps meet at a barrier below)
+          }
+          const unsigned long long now = global_timer_ns();
+          if (t0 == 0) {
+            t0 = now;
+          }
+          else if (now - t0 > WAIT_LIMIT_NS) {
+            *abort_flag = DEV_WAIT_SPLITK;
+            atomicCAS(status, 0u, (uint32_t)DEV_WAIT_SPLITK);
+            break;
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < CB; ++j) {  // ascending CTA order: the result does not depend on timing
+        if (base + j < g.cnt) {
+          __stcg(src + (j * 2 + (base + j == 0 ? 1 : 0)) * (MP * 128), 0u);  // consumed: back to zero for the next launch
+          sum += decode_partial(w[j]);
+        }
+      }
+    }
+    if constexpr (OUT_F32) {
+      reinterpret_cast<float*>(C_out)[(size_t)m * N + (size_t)g.nb * 128 + n] = sum;
+    }
+    else {
+      // largest magnitude of the row, NaN passed over unless there is nothing else (as fmaxf does)
+      const float a  = fabsf(sum);
+      const int   mx = __reduce_max_sync(0xffffffffu, a == a ? __float_as_int(a) : -1);
+      if (lane == 0) {
+        row_max[turn][rw] = __int_as_float(mx);
+      }
+      asm volatile("bar.sync 2, 128;" ::: "memory");  // (alternating rows of row_max: one barrier per row)
+      const float amax = fmaxf(fmaxf(row_max[turn][0], row_max[turn][1]), fmaxf(row_max[turn][2], row_max[turn][3]));
+      const float inv  = amax > 0.0f ? __fdiv_rn(448.0f, amax) : 0.0f;
+      reinterpret_cast<uint8_t*>(C_out)[(size_t)m * N + (size_t)g.nb * 128 + n] = (uint8_t)__nv_cvt_float_to_fp8(sum * inv, __NV_SATFINITE, __NV_E4M3);
+      if (n == 0) {
+        C_s[(size_t)g.nb * M + m] = __fdiv_rn(amax, 448.0f);
+      }
+    }
+  }
+}
+
 // CLUSTER = false: stream-K over all weight blocks, partial tiles through the caller's scratch (above).
 // CLUSTER = true : one thread-block cluster per output group; CTA r of the C in the cluster takes the r-th
 //   slice of the group's K range, and the partial tiles are added through distributed shared memory as a
@@ -515,8 +595,9 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
   // Set-up (barriers, tensor memory, descriptor prefetch) touched no global memory: it may overlap the tail
   // of the previous kernel on the stream, and the next kernel may begin its own set-up from here on.
   pdl_launch_dependents();
-  if (warp != 0) {
-    pdl_wait();  // warp 0 waits below, as a whole: a waiting lane holds up the other lanes of its warp
+  const bool promotes = warp >= EPI_WARP0 && warp < EPI_WARP0 + promo_warps(MP);
+  if (warp != 0 && !promotes) {
+    pdl_wait();  // warp 0 waits below, as a whole: a waiting lane holds up the other lanes of its warp; so do the promotion warps
   }
   PROF_CTA(1);
 
@@ -648,20 +729,32 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
     constexpr int SE = CH * MP / PT;  // elements per thread
     static_assert(SE * PT == CH * MP, "a chunk of scale products must divide among the promotion threads");
     float*        sc = reinterpret_cast<float*>(smem + L::OFF_SC);
-    float         st[SE];
-    auto fetch_chunk = [&](uint32_t chunk) {
+    float         st[SE], st_b[SE];
+    uint32_t      st_a[SE];  // where the activation scale is, NONE: element not used
+    constexpr uint32_t NONE = 0xffffffffu;
+    auto fetch_weight_scales = [&](uint32_t chunk) {
 #pragma unroll
       for (int i = 0; i < SE; ++i) {
         const uint32_t e   = (uint32_t)et + (uint32_t)PT * (uint32_t)i;
         const uint32_t itx = chunk * CH + e / MP;
         const int      m   = (int)(e % MP);
-        float          v   = 0.0f;
+        st_a[i]            = NONE;
         if (itx < run && m < M) {
           const uint32_t uu = itx < len0 ? u_begin + itx : v_begin + (itx - len0);
-          v = __fmul_rn(__ldg(A_s + (size_t)(uu % (uint32_t)KB) * M + m), __ldg(B_s + uu));
+          st_a[i]           = (uu % (uint32_t)KB) * (uint32_t)M + (uint32_t)m;
+          st_b[i]           = __ldg(B_s + uu);
         }
-        st[i] = v;
       }
+    };
+    auto fetch_products = [&]() {
+#pragma unroll
+      for (int i = 0; i < SE; ++i) {
+        st[i] = st_a[i] != NONE ? __fmul_rn(__ldg(A_s + st_a[i]), st_b[i]) : 0.0f;
+      }
+    };
+    auto fetch_chunk = [&](uint32_t chunk) {
+      fetch_weight_scales(chunk);
+      fetch_products();
     };
     auto store_chunk = [&]() {
 #pragma unroll
@@ -669,7 +762,17 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
         sc[et + PT * i] = st[i];
       }
     };
-    fetch_chunk(0);
+    // The scales of static weights and the index arithmetic do not wait for the previous kernel of the stream; with both
+    // behind the wait the first products were ready 1.25 us after the release, later than the first partial.
+    if (early_weights) {
+      fetch_weight_scales(0);
+      pdl_wait();
+    }
+    else {
+      pdl_wait();
+      fetch_weight_scales(0);
+    }
+    fetch_products();
     store_chunk();
     epilogue_bar_sync<PT>();
     if (run > (uint32_t)CH) {
@@ -949,10 +1052,28 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
           }
         }
         bool alive = true;
+        if constexpr (MP <= 16) {
+          // Groups with many contributors: a row per CTA and its four warps.  (The choice is a property of the group: every
+          // contributor makes the same one.)  A warp per row takes eight contributors at a time, so it is as good up to
+          // eight, and up to sixteen where the four warps would have more than one row to do.
+          max_cnt = 0;
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            if (k < n_pend && g[k].cnt > (M <= g[k].cnt ? 8 : 16)) {
+              const int j0 = (int)blockIdx.x - g[k].c_lo;
+              if (j0 < M) {
+                wait_contributors<MP>(g[k], partials, j0, rw * 32, lane, abort_flag, status);
+                reduce_split_group_rows<MP, OUT_F32, 24>(g[k], j0, rw, bars->row_max, partials, C_out, C_s, M, N, lane, abort_flag, status);
+              }
+              g[k].mine = false;
+            }
+            max_cnt = g[k].mine ? max(max_cnt, g[k].cnt) : max_cnt;
+          }
+        }
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
           if (alive && g[k].mine) {
-            alive = wait_contributors<MP>(g[k], partials, lane, abort_flag, status);
+            alive = wait_contributors<MP>(g[k], partials, g[k].gw, 127, lane, abort_flag, status);
           }
         }
         if (alive && (g[0].mine || g[1].mine)) {

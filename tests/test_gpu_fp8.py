@@ -103,6 +103,19 @@ def test_decode_kernel_ragged_m(capi, oracle, cuda, M, NK):
     check_against_oracle(oracle, *case, gq, gs, gf)
 
 
+@pytest.mark.parametrize("M", [1, 3, 9, 10, 16])
+@pytest.mark.parametrize("NK", [(19072, 1024), (19072, 1152), (19072, 2048), (19072, 2176), (19200, 3328), (19072, 6400)])
+def test_left_over_groups_with_many_contributors(capi, oracle, cuda, M, NK):
+    # 149 or 150 groups: one or two left-over groups in pieces of one K-block, 8, 9, 16, 17, 26 and 50 contributors: both
+    # sides of the choice between a warp and four warps per row, and more contributors than are in flight at a time
+    N, K = NK
+    case = make_case(oracle, 47 + M, M, N, K)
+    gq, gs, gf = gpu_mm(capi, cuda, *case)
+    check_against_oracle(oracle, *case, gq, gs, gf)
+    gq2, gs2, gf2 = gpu_mm(capi, cuda, *case)  # and the words went back to zero
+    assert np.array_equal(gq, gq2) and np.array_equal(gs, gs2) and np.array_equal(gf, gf2)
+
+
 @pytest.mark.parametrize("M", [1, 16, 64])
 @pytest.mark.parametrize("NK", QWEN3_4B)
 def test_qwen3_4b_decode_shapes(capi, oracle, cuda, M, NK):
