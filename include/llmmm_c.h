@@ -112,10 +112,10 @@ int llmmm_fp8_blockwise_mm_e4m3out_gather(const void*    A,
  *   h[m, i] = silu(acc[m, i]) * acc[m, I + i],  silu(x) = x / (1 + exp(-x))   (fp32)
  *   H [M, I] e4m3 and H_scale_t [(I/128), M]: h quantised in 1x128 groups along I by the same rule as C above,
  *   which is the A / A_scale_t format of the down projection that consumes it.
- * Requires I%128 == 0, K%128 == 0, any M >= 1.  M > 64 runs one fused kernel (256-row tiles).  M <= 64 runs the
+ * Requires I%128 == 0, K%128 == 0, any M >= 1.  M > 64 runs one fused kernel (128- or 256-row tiles).  M <= 64 runs the
  * weight-streaming decode kernel into scratch followed by a small SwiGLU + quantisation kernel, provided the
  * registered scratch (llmmm_set_workspace) has llmmm_fp8_swiglu_workspace_bytes(M, I, K) bytes; otherwise the
- * 256-row kernel runs for small M too (same results up to the order of fp32 sums, several times slower). */
+ * fused kernel runs for small M too (same results up to the order of fp32 sums, several times slower). */
 int llmmm_fp8_blockwise_mm_swiglu_e4m3out(const void*    A,
                                           const float*   A_scale_t,
                                           const void*    B_gate_up_t,
@@ -143,10 +143,12 @@ size_t llmmm_fp8_swiglu_workspace_bytes(int M, int I, int K);
  *   positions [M] int32 (rows of the angle tables), cos_table / sin_table [table_rows, 64] fp32, weights [128] fp32.
  *   A position outside [0, table_rows) is clamped to the nearest row (no access outside the tables is made) and
  *   recorded: llmmm_check_status then returns LLMMM_ERR_DEVICE_WAIT with code 0x201.
- * Requires K%128 == 0, any M >= 1; tables, weights, A, B_t and C 16-byte aligned.  M > 64 runs one fused kernel
+ * Requires K%128 == 0, any M >= 1; tables, weights, A, B_t and C 16-byte aligned.  M > 128 runs one fused kernel
  * (256-row tiles, always whole: registered scratch is not used).  M <= 64 runs the
  * weight-streaming decode kernel into scratch followed by a small kernel, provided the registered scratch has
- * llmmm_fp8_qk_norm_rope_workspace_bytes(M, N, K) bytes; otherwise the 256-row kernel runs for small M too. */
+ * llmmm_fp8_qk_norm_rope_workspace_bytes(M, N, K) bytes; so does M <= 128 with the 128-row kernel where the plain GEMM
+ * runs on that and the registered scratch has room for the [M, N] accumulator; otherwise the 256-row kernel runs for
+ * small M too. */
 int llmmm_fp8_blockwise_mm_qk_norm_rope_e4m3out(const void*    A,
                                                 const float*   A_scale_t,
                                                 const void*    B_t,

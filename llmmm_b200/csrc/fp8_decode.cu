@@ -44,6 +44,7 @@
 #include <mutex>
 #include <vector>
 
+#include "group_row.cuh"
 #include "host_common.h"
 #include "sm100.cuh"
 
@@ -207,28 +208,6 @@ __device__ __forceinline__ uint4 ld_partial4(const uint32_t* p)
   uint4 v;
   asm volatile("ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
-}
-
-// One finished row of one 128-column output group, four columns per lane of one warp: fp32 as it is, or the
-// row's absmax (the bit pattern of a non-negative float orders like the float: one warp-wide integer max), the
-// two divisions of the quantisation rule, four e4m3 bytes per lane and the scale.
-template<bool OUT_F32>
-__device__ __forceinline__ void store_group_row(float4 s, int m, int nb, void* __restrict__ C_out, float* __restrict__ C_s,
-                                                int M, int N, int lane)
-{
-  if constexpr (OUT_F32) {
-    reinterpret_cast<float4*>(reinterpret_cast<float*>(C_out) + (size_t)m * N + (size_t)nb * 128)[lane] = s;
-  }
-  else {
-    const float    mine = fmaxf(fmaxf(fabsf(s.x), fabsf(s.y)), fmaxf(fabsf(s.z), fabsf(s.w)));
-    const float    amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mine)));
-    const float    inv  = amax > 0.0f ? __fdiv_rn(448.0f, amax) : 0.0f;
-    const uint32_t q    = pack_e4m3x4(s.x * inv, s.y * inv, s.z * inv, s.w * inv);
-    reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(C_out) + (size_t)m * N + (size_t)nb * 128)[lane] = q;
-    if (lane == 0) {
-      C_s[(size_t)nb * M + m] = __fdiv_rn(amax, 448.0f);
-    }
-  }
 }
 
 // Cheap wait in front of the reduction of a split group: lane j polls ONE word of contributor j's partial tile (one

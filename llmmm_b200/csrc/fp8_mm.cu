@@ -33,9 +33,11 @@
 //     every store instruction of the warp touch 32 rows); the scale column is
 //     stored directly, it is coalesced.
 #include <cstddef>
+#include <mutex>
 #include <cuda_fp8.h>
 
 #include "host_common.h"
+#include "group_row.cuh"
 #include "pair_walk.cuh"
 #include "sm100.cuh"
 
@@ -1244,6 +1246,424 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
   }
 }
 
+// ------------------------------------------- CTA pairs, 128-row tiles ----
+//
+// For few rows, where tiles of 256 rows would be half empty or too few: here a pair shares a 128x256 tile
+// (tcgen05.mma.cta_group::2 with M = 128).  CTA r loads 64 rows of A_q and 128 of B_q (24 KB per K-block, seven stages: the weight stream from HBM is
+// the bound, 16 KB per SM every 364 ns).  Its 64 output rows lie in tensor memory twice: lanes 0-63 hold the tile's first
+// 128 columns, lanes 64-127 the second 128, so a partial is 128 columns wide and there are four partial stages.  Eight
+// promotion warps: quarter q drains lanes 32 q .. (rows 32 (q & 1) .., scale group q / 2), and the two warps of a quarter
+// take 64 columns each; they meet at a 64-thread barrier for the row maxima.
+// With few tiles a tile is cut along K among the 2..4 pairs of a larger cluster, and their partial tiles are added through
+// distributed shared memory as a reduce-scatter: the s CTAs that hold the same 64 rows stage their partials in their
+// idle rings, send every other one its share of the rows with one bulk copy, and each adds its rows in K order, one
+// warp per row and scale group.  (Through global scratch, where the pair that arrives last adds everything, the s
+// chunks come in through one pair of SMs: 5.5 us of a 12.1 us launch at 100x2560x4096 with four ways.)
+// EPI_SWIGLU (a tile is 128 gate and the 128 up columns, gate rows of the weight in the leader, up rows in its partner) and
+// EPI_GATHER finish their tiles the same way, one warp per row and group, also when a tile is not cut.  (That costs about
+// 2.5 us for 64 rows.  EPI_ROPE in this form took 19 us for 100x6144x2560, more than the 256-row kernel's 16 us: the
+// hook's arithmetic is issue-bound with four values per lane.)
+namespace fp8p128 {
+constexpr int      BM         = 128;  // per pair; 64 rows per CTA
+constexpr int      BN         = 256;
+constexpr int      BK         = 128;
+constexpr int      UMMA_K     = 32;
+constexpr uint32_t STAGES     = 7;
+constexpr int      THREADS    = 384;
+constexpr int      REGS_CTRL  = 56;
+constexpr int      REGS_PROMO = 224;
+static_assert(128 * REGS_CTRL + 256 * REGS_PROMO <= THREADS * 168, "setmaxnreg split exceeds the CTA's registers");
+constexpr uint32_t A_BYTES    = 64 * BK;
+constexpr uint32_t B_BYTES    = 128 * BK;
+constexpr uint32_t STAGE_TX   = 2 * (A_BYTES + B_BYTES);
+constexpr int      SC_KB      = 4;   // ring of scale operands as in the 256-row kernel: 64 A scales and two B scales
+constexpr int      SC_SLOTS   = 4;
+constexpr int      SC_ROW     = 68;  // floats per K-block, padded to 16 bytes
+constexpr uint32_t OFF_B      = STAGES * A_BYTES;
+constexpr uint32_t OFF_STG    = OFF_B + STAGES * B_BYTES;  // eight staging tiles of 4 KB (e4m3 output: 2 KB of them)
+constexpr uint32_t OFF_XCH    = OFF_STG + 8 * 4096;        // 256 floats: row maxima of the column halves
+constexpr uint32_t OFF_SC     = OFF_XCH + 1024;
+constexpr uint32_t OFF_BAR    = OFF_SC + SC_SLOTS * SC_KB * SC_ROW * 4;
+constexpr uint32_t SMEM_BYTES = OFF_BAR + 512 + 1024;
+static_assert(SMEM_BYTES <= 232448, "shared memory of an SM");
+constexpr int      MAX_WAYS   = 4;     // clusters of up to eight CTAs
+constexpr uint32_t ROW_BYTES  = BN * 4;  // a row of a staged partial tile, its 16-byte chunks XOR-swizzled by the row
+constexpr uint32_t OFF_RCV    = 64 * ROW_BYTES;
+static_assert(OFF_RCV + (64 + MAX_WAYS) * ROW_BYTES <= OFF_STG, "partial tiles must fit into the idle ring");
+}  // namespace fp8p128
+
+struct Fp8Pair128Bars {
+  uint64_t full[fp8p128::STAGES];        // used in the leader CTA
+  uint64_t done[fp8p128::STAGES];        // both CTAs (multicast commit): ring slot free, partial ready
+  uint64_t part_empty[4];                // used in the leader CTA, 16 arrivals
+  uint64_t sc_full[fp8p128::SC_SLOTS];   // 32 arrivals
+  uint64_t sc_empty[fp8p128::SC_SLOTS];  // 8 arrivals
+  uint64_t red;                          // the other CTAs' partials of this CTA's rows have landed (counted in bytes)
+  uint32_t tmem_base;
+  uint32_t abort_flag;
+};
+static_assert(sizeof(Fp8Pair128Bars) <= 512, "barriers");
+
+template<int EPI>
+__global__ void __launch_bounds__(fp8p128::THREADS, 1)
+  fp8_blockwise_gemm_pair_kernel_m128(const __grid_constant__ CUtensorMap tm_a,
+                                      const __grid_constant__ CUtensorMap tm_b,
+                                      const __grid_constant__ CUtensorMap tm_c,  // C as rows of bytes, boxes of 32 rows x 64 (fp32: 128) bytes
+                                      const float* __restrict__ A_s,
+                                      const float* __restrict__ B_s,
+                                      void* __restrict__ C_out,
+                                      float* __restrict__ C_s,
+                                      int       M,
+                                      int       N,
+                                      int       K,
+                                      const __grid_constant__ GatherDst gather,
+                                      uint32_t* status)
+{
+  using namespace fp8p128;
+  constexpr bool OUT_F32 = EPI == EPI_F32, SWIGLU = EPI == EPI_SWIGLU;
+  constexpr bool BY_ROW  = EPI != EPI_F32 && EPI != EPI_E4M3;  // rows are finished by warps even if the tile is not cut
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  Fp8Pair128Bars*    bars       = reinterpret_cast<Fp8Pair128Bars*>(smem + OFF_BAR);
+  float*             sc_ring    = reinterpret_cast<float*>(smem + OFF_SC);
+  volatile uint32_t* abort_flag = &bars->abort_flag;
+
+  const int      warp     = threadIdx.x >> 5;
+  const int      lane     = threadIdx.x & 31;
+  uint32_t       c_size;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(c_size));
+  const uint32_t c_rank   = cluster_ctarank();
+  const uint32_t rank     = c_rank & 1;   // in the pair
+  const uint32_t leader   = c_rank & ~1u;
+  const uint32_t ways     = c_size >> 1;
+  const uint32_t part     = c_rank >> 1;  // this pair's slice of K
+  const int      m_tiles  = (M + BM - 1) / BM;
+  const int      tile     = (blockIdx.x / c_size) / m_tiles;  // 256 columns (SWIGLU: 128 gate and the 128 up columns)
+  const int      m0       = (int)((blockIdx.x / c_size) % m_tiles) * BM + (int)rank * 64;  // this CTA's 64 rows
+  const int      k_blocks = K / BK;
+  const int      kb0      = (int)(part * (uint32_t)k_blocks / ways), kb1 = (int)((part + 1) * (uint32_t)k_blocks / ways);
+  const int      n_groups = N / 128;
+
+  if (threadIdx.x == 0) {
+    for (uint32_t s = 0; s < STAGES; ++s) {
+      mbar_init(&bars->full[s], 1);
+      mbar_init(&bars->done[s], 1);
+    }
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(&bars->part_empty[i], 16);
+    }
+    for (int i = 0; i < SC_SLOTS; ++i) {
+      mbar_init(&bars->sc_full[i], 32);
+      mbar_init(&bars->sc_empty[i], 8);
+    }
+    mbar_init(&bars->red, 1);
+    bars->abort_flag = 0;
+    fence_mbar_init();
+    prefetch_tmap(&tm_a);
+    prefetch_tmap(&tm_b);
+    if constexpr (!BY_ROW) {
+      prefetch_tmap(&tm_c);
+    }
+  }
+  if (warp == 2) {
+    tmem_alloc<512>(&bars->tmem_base);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = bars->tmem_base;
+  // no global memory touched so far: this may overlap the tail of the previous kernel on the stream
+  pdl_launch_dependents();
+  pdl_wait();
+
+  if (warp < 4) {
+    setmaxnreg_dec<REGS_CTRL>();
+    if (warp == 0) {
+      // ---------------------------------------------------- TMA producer --
+      if (lane == 0) {
+        uint32_t s = 0, ph = 0;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          mbar_wait(&bars->done[s], ph ^ 1, DEV_WAIT_SMEM_EMPTY, abort_flag, status);
+          const uint32_t full_leader = mapa_shared(smem_u32(&bars->full[s]), leader);
+          if (rank == 0) {
+            mbar_arrive_expect_tx(&bars->full[s], STAGE_TX);
+          }
+          tma_load_2d_pair(smem + OFF_B + s * B_BYTES, &tm_b, full_leader, kb * BK, SWIGLU ? tile * 128 + (int)rank * N : tile * BN + (int)rank * 128);
+          tma_load_2d_pair(smem + s * A_BYTES, &tm_a, full_leader, kb * BK, m0);
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+      }
+    }
+    else if (warp == 2) {
+      // -------------------------------------------------- scale operands --
+      uint32_t     c   = 0;
+      const float* b_s = B_s + (size_t)(SWIGLU ? tile + (lane & 1) * n_groups : min(tile * 2 + (lane & 1), n_groups - 1)) * k_blocks;
+      for (int kb = kb0; kb < kb1; kb += SC_KB, ++c) {
+        const uint32_t slot = c % SC_SLOTS;
+        mbar_wait(&bars->sc_empty[slot], ((c / SC_SLOTS) & 1) ^ 1, DEV_WAIT_SMEM_EMPTY, abort_flag, status);
+        uint32_t dst = smem_u32(sc_ring) + (slot * SC_KB * SC_ROW + lane) * 4;
+#pragma unroll 1
+        for (int k = kb; k < min(kb + SC_KB, kb1); ++k, dst += SC_ROW * 4) {
+          const float* a_s = A_s + (size_t)k * M;
+          cp_async_4(dst, a_s + min(m0 + lane, M - 1));  // (rows beyond M: any valid scale)
+          cp_async_4(dst + 128, a_s + min(m0 + 32 + lane, M - 1));
+          if (lane < 2) {
+            cp_async_4(dst + 256, b_s + k);
+          }
+        }
+        cp_async_arrive(&bars->sc_full[slot]);
+      }
+      cp_async_wait_all();
+    }
+    else if (lane == 0 && rank == 0) {
+      // ------------------------------------ two MMA issuers (leader only) --
+      constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, BM, BN);
+      const uint32_t     total = (uint32_t)(kb1 - kb0);
+      for (uint32_t it = warp == 1 ? 0u : 1u; it < total; it += 2) {
+        const uint32_t s = it % STAGES;
+        // (the stage's previous K-block is this thread's own: its phases are met in order)
+        mbar_wait(&bars->part_empty[it & 3], ((it >> 2) & 1) ^ 1, DEV_WAIT_TMEM_EMPTY, abort_flag, status);
+        mbar_wait(&bars->full[s], (it / STAGES) & 1, DEV_WAIT_SMEM_FULL, abort_flag, status);
+        tc_fence_after_sync();
+        const uint64_t da = make_smem_desc_sw128(smem_u32(smem + s * A_BYTES), 0, 1024);
+        const uint64_t db = make_smem_desc_sw128(smem_u32(smem + OFF_B + s * B_BYTES), 0, 1024);
+#pragma unroll
+        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+          tc_mma_f8_pair(tmem_base + (it & 3) * 128, da + (uint64_t)((kk * UMMA_K) >> 4), db + (uint64_t)((kk * UMMA_K) >> 4), idesc, kk != 0);
+        }
+        tc_commit_pair(&bars->done[s], (uint16_t)(3u << leader));
+      }
+    }
+    if (ways > 1) {
+      __syncwarp();
+      cluster_sync_all();  // every CTA's ring is idle and its staged partial complete
+    }
+  }
+  else {
+    setmaxnreg_inc<REGS_PROMO>();
+    // ------------------------------------------- promotion + epilogue ----
+    const int      quarter      = warp & 3;         // tensor-memory lane quarter this warp may read
+    const int      half         = (warp - 4) >> 2;  // which 64 columns of the scale group
+    const int      m            = m0 + (quarter & 1) * 32 + lane;
+    const uint32_t t_mine       = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 64);
+    const uint32_t bars_at      = smem_u32(bars);
+    const uint32_t abort_at     = smem_u32(&bars->abort_flag);
+    const uint32_t empty_leader = mapa_shared(smem_u32(&bars->part_empty[0]), leader);
+    const uint32_t sc_mine      = smem_u32(sc_ring) + ((quarter & 1) * 32 + lane) * 4;
+    const uint32_t sc_b         = (64 - (quarter & 1) * 32 - lane + (quarter >> 1)) * 4;
+    uint8_t*       stg          = smem + OFF_STG + (warp - 4) * 4096;
+    uint32_t       it = 0, st = 0, st_ph = 0, sc_slot = 0, sc_ph = 0;
+    {
+      const int  ng   = tile * 2 + (quarter >> 1);
+      const bool m_ok = m < M;
+      const bool g_ok = ng < n_groups;
+      float      acc[64];
+#pragma unroll
+      for (int i = 0; i < 64; ++i) {
+        acc[i] = 0.0f;
+      }
+      for (int left = kb1 - kb0; left > 0; left -= SC_KB) {
+        mbar_wait_at(bars_at + (uint32_t)offsetof(Fp8Pair128Bars, sc_full) + sc_slot * 8, sc_ph, DEV_WAIT_SMEM_FULL, abort_at, status);
+        uint32_t       sc_addr = sc_mine + sc_slot * (SC_KB * SC_ROW * 4);
+        const uint32_t sc_end  = sc_addr + min(left, SC_KB) * (SC_ROW * 4);
+#pragma unroll 1
+        for (; sc_addr != sc_end; sc_addr += SC_ROW * 4) {
+          // one fp32 rounding of the scale product, as in the reference
+          float sc = __fmul_rn(lds_f32(sc_addr), lds_f32(sc_addr + sc_b));
+          mbar_wait_at(bars_at + (uint32_t)offsetof(Fp8Pair128Bars, done) + st * 8, st_ph, DEV_WAIT_TMEM_FULL, abort_at, status);
+          tc_fence_after_sync();
+          uint32_t v0[32], v1[32];
+          tmem_ld_32x32b_x32(t_mine + (it & 3) * 128, v0);
+          tmem_ld_32x32b_x32(t_mine + (it & 3) * 128 + 32, v1);
+          tmem_ld_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive_cluster_relaxed(empty_leader + (it & 3) * 8);
+          }
+          asm volatile("" : "+f"(sc));  // the arithmetic stays behind the hand-back
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            ffma2(acc[i], acc[i + 1], v0[i], v0[i + 1], sc);
+          }
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            ffma2(acc[32 + i], acc[32 + i + 1], v1[i], v1[i + 1], sc);
+          }
+          ++it;
+          if (++st == STAGES) {
+            st = 0;
+            st_ph ^= 1;
+          }
+        }
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive_at(bars_at + (uint32_t)offsetof(Fp8Pair128Bars, sc_empty) + sc_slot * 8);
+        }
+        if (++sc_slot == SC_SLOTS) {
+          sc_slot = 0;
+          sc_ph ^= 1;
+        }
+      }
+
+      if (BY_ROW || ways > 1) {
+        const uint32_t share = (64 + ways - 1) / ways;  // rows per CTA
+        auto rows_of = [&](uint32_t o) {                 // rows of these 64 that CTA `o` of the ways finishes
+          const int lo = (int)(o * share), hi = min(min(lo + (int)share, 64), M - m0);
+          return (uint32_t)max(hi - lo, 0);
+        };
+        const uint32_t my_rows = rows_of(part);
+        const int      rr      = (quarter & 1) * 32 + lane;
+        uint8_t*       row     = smem + rr * ROW_BYTES;
+        const int      chunk0  = (quarter >> 1) * 32 + half * 16;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          *reinterpret_cast<float4*>(row + (((chunk0 + i) ^ (rr & 7)) << 4)) = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
+        }
+        if (ways == 1) {
+          asm volatile("bar.sync 1, 256;" ::: "memory");
+        }
+        else {
+        fence_proxy_async_smem();  // the bulk copies below read what was just written
+        if (threadIdx.x == 128) {
+          mbar_arrive_expect_tx(&bars->red, (ways - 1) * my_rows * ROW_BYTES);
+        }
+        cluster_sync_all();
+        if (warp == 4 && (uint32_t)lane < ways && (uint32_t)lane != part && rows_of((uint32_t)lane) != 0) {  // one lane per destination
+          const uint32_t o = (uint32_t)lane;
+          bulk_copy_to_peer(mapa_shared(smem_u32(smem + OFF_RCV + part * share * ROW_BYTES), 2 * o + rank), smem + o * share * ROW_BYTES,
+                            rows_of(o) * ROW_BYTES, mapa_shared(smem_u32(&bars->red), 2 * o + rank));
+        }
+        __syncwarp();
+        if (my_rows != 0) {
+          mbar_wait(&bars->red, 0, DEV_WAIT_SPLITK, abort_flag, status);
+        }
+        }
+        // a row's 128 values of group `grp` of the tile, four per lane
+        auto row_sum = [&](uint32_t q, uint32_t grp) {
+          const uint32_t r   = part * share + q;  // row of this CTA's 64
+          const uint32_t at  = (((grp * 32 + (uint32_t)lane) ^ (r & 7)) << 4);
+          float4         sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          for (uint32_t o = 0; o < ways; ++o) {  // in the order of the K slices: the result does not depend on timing
+            const uint8_t* src = o == part ? smem + r * ROW_BYTES : smem + OFF_RCV + (o * share + q) * ROW_BYTES;
+            const float4   p   = *reinterpret_cast<const float4*>(src + at);
+            sum.x += p.x;
+            sum.y += p.y;
+            sum.z += p.z;
+            sum.w += p.w;
+          }
+          return sum;
+        };
+        // four rows (and groups) per warp at a time: their chains of loads, maxima and divisions overlap
+        const uint32_t items = SWIGLU ? my_rows : 2 * my_rows;
+        for (uint32_t q0 = (uint32_t)(warp - 4); q0 < items; q0 += 32) {
+          float4 sum[4];
+          int    row_of[4], group_of[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t q = min(q0 + 8 * j, items - 1);
+            row_of[j]        = m0 + (int)(part * share + (SWIGLU ? q : q >> 1));
+            group_of[j]      = q0 + 8 * j >= items ? n_groups : SWIGLU ? tile : tile * 2 + (int)(q & 1);
+            sum[j]           = row_sum(SWIGLU ? q : q >> 1, SWIGLU ? 0u : q & 1);
+            if constexpr (SWIGLU) {
+              const float4 up = row_sum(q, 1u);
+              sum[j].x        = __fdividef(sum[j].x, 1.0f + __expf(-sum[j].x)) * up.x;
+              sum[j].y        = __fdividef(sum[j].y, 1.0f + __expf(-sum[j].y)) * up.y;
+              sum[j].z        = __fdividef(sum[j].z, 1.0f + __expf(-sum[j].z)) * up.z;
+              sum[j].w        = __fdividef(sum[j].w, 1.0f + __expf(-sum[j].w)) * up.w;
+            }
+          }
+          if constexpr (EPI == EPI_GATHER) {
+            for (int d = 0; d < gather.n; ++d) {
+              store_group_rows<false>(sum, row_of, group_of, n_groups, gather.c[d] + gather.col0, gather.cs[d] + (size_t)(gather.col0 / 128) * M, M,
+                                      gather.ld, lane);
+            }
+          }
+          else {
+            store_group_rows<OUT_F32>(sum, row_of, group_of, n_groups, C_out, C_s, M, N, lane);
+          }
+        }
+      }
+      else if constexpr (BY_ROW) {
+        // (finished above)
+      }
+      else if constexpr (OUT_F32) {
+        // two passes of 32 columns through the warp's staging tile, each leaving as one TMA store (whole 128-byte rows)
+#pragma unroll
+        for (int ps = 0; ps < 2; ++ps) {
+          if (lane == 0) {
+            tma_store_wait_read<0>();  // the previous store has read the staging tile
+          }
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            *reinterpret_cast<float4*>(stg + lane * 128 + ((i ^ (lane & 7)) << 4)) =
+              make_float4(acc[32 * ps + 4 * i], acc[32 * ps + 4 * i + 1], acc[32 * ps + 4 * i + 2], acc[32 * ps + 4 * i + 3]);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && g_ok && m - lane < M) {
+            tma_store_2d(&tm_c, stg, ng * 512 + half * 256 + ps * 128, m - lane);
+            tma_store_commit();
+          }
+        }
+      }
+      else {
+        float a4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int i = 0; i < 64; ++i) {
+          a4[i & 3] = fmaxf(a4[i & 3], fabsf(acc[i]));
+        }
+        float amax = fmaxf(fmaxf(a4[0], a4[1]), fmaxf(a4[2], a4[3]));
+        // the other 64 columns of the group belong to the other warp of the quarter
+        float* xch = reinterpret_cast<float*>(smem + OFF_XCH);
+        xch[half * 128 + quarter * 32 + lane] = amax;
+        if (lane == 0) {
+          tma_store_wait_read<0>();  // the store of the previous tile has read the staging tile
+        }
+        asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
+        amax = fmaxf(amax, xch[(half ^ 1) * 128 + quarter * 32 + lane]);
+        const float scale     = __fdiv_rn(amax, 448.0f);
+        const float scale_inv = amax > 0.0f ? __fdiv_rn(448.0f, amax) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint4 o;
+          o.x = pack_e4m3x4(acc[16 * i + 0] * scale_inv, acc[16 * i + 1] * scale_inv, acc[16 * i + 2] * scale_inv, acc[16 * i + 3] * scale_inv);
+          o.y = pack_e4m3x4(acc[16 * i + 4] * scale_inv, acc[16 * i + 5] * scale_inv, acc[16 * i + 6] * scale_inv, acc[16 * i + 7] * scale_inv);
+          o.z = pack_e4m3x4(acc[16 * i + 8] * scale_inv, acc[16 * i + 9] * scale_inv, acc[16 * i + 10] * scale_inv, acc[16 * i + 11] * scale_inv);
+          o.w = pack_e4m3x4(acc[16 * i + 12] * scale_inv, acc[16 * i + 13] * scale_inv, acc[16 * i + 14] * scale_inv, acc[16 * i + 15] * scale_inv);
+          *reinterpret_cast<uint4*>(stg + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4)) = o;
+        }
+        if (m_ok && g_ok && half == 0) {
+          C_s[(size_t)ng * M + m] = scale;
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && g_ok && m - lane < M) {
+          tma_store_2d(&tm_c, stg, ng * 128 + half * 64, m - lane);
+          tma_store_commit();
+        }
+      }
+    }
+    if (lane == 0) {
+      tma_store_wait_read<0>();  // shared memory must outlive the last store's read of it
+    }
+  }
+
+  // no CTA may leave while another one can still signal its barriers, read its tiles or write its rows
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();
+  if (warp == 2) {
+    tc_fence_after_sync();
+    tmem_dealloc<512>(tmem_base);
+  }
+}
+
 template<int EPI>
 static int launch_fp8_pair_epi(const void*       A,
                                const float*      A_s,
@@ -1294,6 +1714,124 @@ static int launch_fp8_pair_epi(const void*       A,
   return LLMMM_OK;
 }
 
+// How many clusters of 2 * ways CTAs of the 128-row pair kernel the device can hold at once (an occupancy query, cached).
+static int pair128_capacity(const DeviceInfo* info, int ways)
+{
+  static std::mutex           mu;
+  static int                  cache[64][fp8p128::MAX_WAYS + 1];
+  static bool                 known[64][fp8p128::MAX_WAYS + 1];
+  std::lock_guard<std::mutex> lock(mu);
+  if (!known[info->device][ways]) {
+    int clusters = 0;
+    if (cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_E4M3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES)
+        == cudaSuccess) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim            = dim3((unsigned)(2 * ways * (info->sm_count / (2 * ways))));
+      cfg.blockDim           = dim3(fp8p128::THREADS);
+      cfg.dynamicSmemBytes   = fp8p128::SMEM_BYTES;
+      cudaLaunchAttribute attr[1];
+      attr[0].id               = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)(2 * ways);
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs                = attr;
+      cfg.numAttrs             = 1;
+      if (cudaOccupancyMaxActiveClusters(&clusters, fp8_blockwise_gemm_pair_kernel_m128<EPI_E4M3>, &cfg) != cudaSuccess) {
+        clusters = 0;
+      }
+    }
+    cudaGetLastError();
+    cache[info->device][ways] = clusters;
+    known[info->device][ways] = true;
+  }
+  return cache[info->device][ways];
+}
+
+// Pairs that share a tile along K: as many as leave every tile a resident cluster, and only where the K-blocks saved
+// (0.36 us each) are worth the exchange (2.5 us).
+static int pair128_ways(const DeviceInfo* info, int M, int N, int K)
+{
+  const int tiles    = ((M + fp8p128::BM - 1) / fp8p128::BM) * ((N + fp8p128::BN - 1) / fp8p128::BN);
+  const int k_blocks = K / fp8p128::BK;
+  for (int ways = fp8p128::MAX_WAYS; ways >= 2; --ways) {
+    if (2 * ways * tiles <= info->sm_count && k_blocks - (k_blocks + ways - 1) / ways > 7 && pair128_capacity(info, ways) >= tiles) {
+      return ways;
+    }
+  }
+  return 1;
+}
+
+// Whether a problem that is the pair kernels' runs with 128-row tiles.  Up to 128 rows always.  Above, a 128-row tile has
+// half the work at about 0.6 of the time per K-block (0.3-0.36 against 0.55 us), so it wins where its tiles (cut along K or
+// not) fit on the pairs at once and those of 256 rows leave pairs idle or are cut; the fixed costs are 3.8 and 5 us, cutting
+// costs 2.5 us here and about 3 + 1.5 per way there.  Measured, 256-row against 128-row tiles: 256x2560x9728 23.5 / 15.5 us,
+// 256x6144x2560 15.4 / 9.9, 512x4096x4096 18.9 / 13.5, 700x2560x4096 18.7 / 13.4.  Beyond 768 rows only tiles that are
+// cut: callers are told (llmmm_split_launch_count, llmmm_c.h) that the last wave of such a problem is cut along K when
+// scratch is registered.
+static bool use_pair128(const DeviceInfo* info, int M, int N, int K)
+{
+  if (M <= fp8p128::BM) {
+    return true;
+  }
+  const int       tiles = ((M + fp8p128::BM - 1) / fp8p128::BM) * ((N + fp8p128::BN - 1) / fp8p128::BN);
+  const Workspace ws    = registered_workspace(info->device);
+  if (tiles > info->max_pairs || ws.ptr == nullptr || ws.bytes < split_workspace_bytes()) {
+    return false;
+  }
+  const int k_blocks = K / fp8p128::BK, ways = pair128_ways(info, M, N, K);
+  if (M > 768 && ways == 1) {
+    return false;
+  }
+  const float     us128    = 0.36f * (float)((k_blocks + ways - 1) / ways) + (ways > 1 ? 2.5f : 0.0f) + 3.8f;
+  const int       tiles256 = ((M + fp8pair::BM - 1) / fp8pair::BM) * ((N + fp8pair::BN - 1) / fp8pair::BN);
+  const SplitPlan plan     = plan_split(info, tiles256, k_blocks, 4, 5, 3, false);
+  const int       longest  = (plan.dp_tiles + plan.pairs - 1) / plan.pairs * k_blocks + (plan.split_pairs > 0 ? plan.split_chunk : 0);
+  const float     us256    = 0.55f * (float)longest + (plan.split_pairs > 0 ? 3.0f + 1.5f * (float)plan.split_s : 0.0f) + 5.0f;
+  return us128 < us256;
+}
+
+// The same choice for the SwiGLU form, which never cuts tiles and does not look at the scratch: 128-row tiles cost 0.36 us
+// per K-block and 6.3 us (the rows included), those of 256 rows 0.6 us per K-block and 6 us.  Measured at 9728 output
+// columns and 100 rows 25.4 us against 28.2 us; 200 rows stay on 256-row tiles, 27.0 us.
+static bool use_pair128_swiglu(const DeviceInfo* info, int M, int I, int K)
+{
+  const int k_blocks = K / fp8p128::BK, P = info->max_pairs;
+  const int waves128 = ((M + fp8p128::BM - 1) / fp8p128::BM * (I / 128) + P - 1) / P;
+  const int waves256 = ((M + fp8pair::BM - 1) / fp8pair::BM * (I / 128) + P - 1) / P;
+  return (float)waves128 * (0.36f * (float)k_blocks + 6.3f) < 0.6f * (float)(waves256 * k_blocks) + 6.0f;
+}
+
+template<int EPI>
+static int launch_fp8_pair128(const void* A, const float* A_s, const void* B, const float* B_s, void* C, float* C_s, int M, int N,
+                              int K, const GatherDst& gather, const DeviceInfo* info, cudaStream_t stream)
+{
+  using namespace fp8p128;
+  CUtensorMap    tm_a, tm_b, tm_c = {};
+  const uint64_t row_bytes = (uint64_t)N * (EPI == EPI_F32 ? 4 : 1), b_rows = (uint64_t)N * (EPI == EPI_SWIGLU ? 2 : 1);
+  if (!make_tmap_2d(&tm_a, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)M, (uint64_t)K, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B)
+      || !make_tmap_2d(&tm_b, B, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, b_rows, (uint64_t)K, BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)
+      || ((EPI == EPI_F32 || EPI == EPI_E4M3)
+          && !make_tmap_2d(&tm_c, C, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, row_bytes, (uint64_t)M, row_bytes, EPI == EPI_F32 ? 128 : 64, 32,
+                           EPI == EPI_F32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B))) {
+    return LLMMM_ERR_CUDA;
+  }
+  static thread_local bool attr_set[64] = {};
+  if (!attr_set[info->device]) {
+    LLMMM_CUDA_TRY(cudaFuncSetAttribute(
+      fp8_blockwise_gemm_pair_kernel_m128<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
+    attr_set[info->device] = true;
+  }
+  const int ways  = EPI == EPI_SWIGLU ? 1 : pair128_ways(info, M, N, K);
+  const int tiles = ((M + BM - 1) / BM) * (EPI == EPI_SWIGLU ? N / 128 : (N + BN - 1) / BN);
+  if (ways > 1) {
+    g_split_launches.fetch_add(1);
+  }
+  LLMMM_CUDA_TRY(launch_pdl(fp8_blockwise_gemm_pair_kernel_m128<EPI>, dim3((unsigned)(2 * ways * tiles)), dim3(THREADS), SMEM_BYTES,
+                            stream, (unsigned)(2 * ways), tm_a, tm_b, tm_c, A_s, B_s, C, C_s, M, N, K, gather, info->status));
+  g_launches.fetch_add(1);
+  return LLMMM_OK;
+}
+
 template<bool OUT_F32>
 static int launch_fp8_pair(const void* A, const float* A_s, const void* B, const float* B_s, void* C, float* C_s, int M,
                            int N, int K, const DeviceInfo* info, cudaStream_t stream)
@@ -1315,6 +1853,9 @@ static int launch_fp8_swiglu(const void*       A,
                              cudaStream_t      stream)
 {
   using namespace fp8pair;
+  if (use_pair128_swiglu(info, M, I, K)) {
+    return launch_fp8_pair128<EPI_SWIGLU>(A, A_s, B, B_s, H, H_s, M, I, K, GatherDst{}, info, stream);
+  }
   CUtensorMap tm_a, tm_b;
   if (!make_tmap_2d(&tm_a, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)M, (uint64_t)K, BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)
       || !make_tmap_2d(&tm_b, B, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)2 * I, (uint64_t)K, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B)) {
@@ -1356,6 +1897,9 @@ static int launch_fp8_gather(const void*       A,
                              cudaStream_t      stream)
 {
   using namespace fp8pair;
+  if (fp8_use_pair_kernel(info, M, N, K) && use_pair128(info, M, N, K)) {  // (what the plain entry point runs for the same shard, so the bytes agree)
+    return launch_fp8_pair128<EPI_GATHER>(A, A_s, B, B_s, nullptr, nullptr, M, N, K, dst, info, stream);
+  }
   CUtensorMap tm_a, tm_b;
   if (!make_tmap_2d(&tm_a, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)M, (uint64_t)K, BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)
       || !make_tmap_2d(&tm_b, B, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)N, (uint64_t)K, BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)) {
@@ -1395,6 +1939,9 @@ static int launch_fp8(const void*  A,
     return LLMMM_ERR_UNSUPPORTED;
   }
   if (fp8_use_pair_kernel(info, M, N, K)) {
+    if (use_pair128(info, M, N, K)) {
+      return launch_fp8_pair128<(OUT_F32 ? EPI_F32 : EPI_E4M3)>(A, A_s, B, B_s, C, C_s, M, N, K, GatherDst{}, info, stream);
+    }
     return launch_fp8_pair<OUT_F32>(A, A_s, B, B_s, C, C_s, M, N, K, info, stream);
   }
   CUtensorMap tm_a, tm_b;
@@ -1433,6 +1980,12 @@ void describe_fp8_plan(const DeviceInfo* info, bool out_f32, int M, int N, int K
   const char* how   = (M > 64 && M <= 128) ? (tuned ? " (kernel choice: measured by llmmm_tune)" : " (kernel choice: default rule)") : "";
   if (pair) {
     using namespace fp8pair;
+    if (use_pair128(info, M, N, K)) {
+      const int tiles = ((M + fp8p128::BM - 1) / fp8p128::BM) * ((N + fp8p128::BN - 1) / fp8p128::BN), ways = pair128_ways(info, M, N, K);
+      snprintf(buf, len, "fp8_blockwise_gemm_pair_kernel_m128<%s>: %d tiles of 128x256, each on %d CTA pair(s) of a cluster that share its %d "
+               "K-blocks and add their partial tiles through distributed shared memory%s", o, tiles, ways, K / fp8p128::BK, how);
+      return;
+    }
     const int       tiles    = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
     const int       k_blocks = K / BK;
     const SplitPlan plan     = plan_split(info, tiles, k_blocks, 4, 5, 3, false);
@@ -1468,6 +2021,10 @@ int warm_fp8_kernels(const DeviceInfo* info)
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_SWIGLU)));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_GATHER)));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_ROPE)));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_E4M3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8cfg::SMEM_BYTES));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8cfg::SMEM_BYTES));
   return warm_decode_kernels(info);
@@ -1757,6 +2314,15 @@ int llmmm_fp8_blockwise_mm_qk_norm_rope_e4m3out(const void*    A,
   }
   if (info->max_pairs < 1) {
     return set_error(LLMMM_ERR_UNSUPPORTED, "this device cannot hold a cluster of two CTAs of the GEMM kernel");
+  }
+  if (M > 64 && M <= fp8p128::BM && fp8_use_pair_kernel(info, M, N, K)) {
+    // 65..128 rows: the 128-row pair kernel into scratch and the small kernel (100x6144x2560: 9.5 + 2.3 us against 16.0 us)
+    const Workspace ws = registered_workspace(info->device);
+    if (ws.ptr != nullptr && ws.bytes >= decode_acc_offset(M, N) + (size_t)M * N * sizeof(float)) {
+      float*    acc = reinterpret_cast<float*>(static_cast<uint8_t*>(ws.ptr) + decode_acc_offset(M, N));
+      const int rc  = launch_fp8_pair128<EPI_F32>(A, A_scale_t, B_t, B_scale_t, acc, nullptr, M, N, K, GatherDst{}, info, s);
+      return rc != LLMMM_OK ? rc : launch_rope_quant(acc, C, C_scale_t, hook, M, N, info->status, s);
+    }
   }
   return launch_fp8_pair_epi<EPI_ROPE>(A, A_scale_t, B_t, B_scale_t, C, C_scale_t, M, N, K, hook, info, s);
 }

@@ -510,9 +510,9 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
 
 // Completion of all MMAs issued so far by this thread arrives on the mbarrier
 // at the same shared-memory offset in both CTAs of the pair.
-__device__ __forceinline__ void tc_commit_pair(uint64_t* bar)
+// (`mask`: the cluster ranks of the pair).
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar, uint16_t mask = 3)
 {
-  const uint16_t mask = 3;
   asm volatile(
     "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
       smem_u32(bar)),

@@ -240,6 +240,24 @@ def test_mid_m_few_tiles_take_the_pair_kernel_with_scratch(capi, oracle, cuda, s
     assert np.abs(gf - gf2).max() <= 4e-6 * np.abs(gf).max()
 
 
+@pytest.mark.parametrize("shape", [(1 + 64, 256, 1024), (127, 384, 2176), (128, 2560, 1280), (100, 6144, 1152), (65, 9472, 512),
+                                   (129, 2560, 2048), (191, 640, 3200), (257, 1280, 2560), (384, 896, 1152), (641, 512, 1280), (1030, 256, 4096)])
+def test_pair_kernel_128_row_tiles(capi, oracle, cuda, shape):
+    # one to four pairs per tile (10 to 74 tiles), rows and column groups beyond the matrix, slices of K of unequal length,
+    # K-blocks that are no multiple of the scale ring's four
+    M, N, K = shape
+    case = make_case(oracle, 48, M, N, K)
+    capi.clear_workspace()
+    gq, gs, gf = gpu_mm(capi, cuda, *case, workspace=False)
+    capi.ensure_workspace(M, N, K)
+    assert "pair_kernel_m128" in capi.describe_plan("fp8", M, N, K)
+    gq2, gs2, gf2 = gpu_mm(capi, cuda, *case)
+    check_against_oracle(oracle, *case, gq2, gs2, gf2)
+    assert np.abs(gf - gf2).max() <= 4e-6 * np.abs(gf).max()
+    gq3, gs3, gf3 = gpu_mm(capi, cuda, *case)
+    assert np.array_equal(gq2, gq3) and np.array_equal(gs2, gs3) and np.array_equal(gf2, gf3)
+
+
 def gpu_c_quant(acc):
     """The output quantisation rule in torch fp32 on the GPU (for full-size property checks)."""
     M, N = acc.shape

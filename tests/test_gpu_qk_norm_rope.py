@@ -148,6 +148,19 @@ def test_decode_sized(capi, oracle, cuda, M):
     check(oracle, c, gq, gs)
 
 
+@pytest.mark.parametrize("M", [65, 128])
+@pytest.mark.parametrize("weights", [True, False])
+def test_65_to_128_rows(capi, oracle, cuda, M, weights):
+    # with scratch: the 128-row pair kernel + the small hook kernel; without, the fused 256-row kernel
+    c = make_case(oracle, 75, M, 16, 4, 1152, weights=weights)
+    capi.clear_workspace()
+    gq, gs = run(capi, cuda, c)
+    check(oracle, c, gq, gs)
+    capi.ensure_workspace(c["M"], c["N"], c["K"])
+    gq2, gs2 = run(capi, cuda, c, launches=2)
+    check(oracle, c, gq2, gs2)
+
+
 def test_argument_errors(capi, cuda):
     c = dict(M=128, N=512, K=256)
     z8 = torch.zeros(128 * 512, dtype=torch.uint8, device=cuda)

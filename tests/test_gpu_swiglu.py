@@ -129,6 +129,17 @@ def test_swiglu_decode_sized(capi, oracle, cuda, M, IK):
     assert np.array_equal(gq2, gq3) and np.array_equal(gs2.view(np.uint32), gs3.view(np.uint32))
 
 
+@pytest.mark.parametrize("shape", [(65, 1152, 384), (128, 9728, 256), (100, 9472, 256), (300, 2560, 512)])
+def test_swiglu_128_row_tiles(capi, oracle, cuda, shape):
+    # the 128-row pair kernel's form: one and two waves of tiles, rows beyond the matrix in either CTA of a pair
+    M, I, K = shape
+    case = make_case(oracle, 96, M, I, K)
+    gq, gs = run(capi, cuda, case, M, I, K)
+    check(oracle, case, gq, gs)
+    gq2, gs2 = run(capi, cuda, case, M, I, K)
+    assert np.array_equal(gq, gq2) and np.array_equal(gs, gs2)
+
+
 @pytest.mark.parametrize("M", [33, 64])
 def test_decode_call_after_a_hook_call_with_fewer_rows(capi, oracle, cuda, M):
     # The hook's accumulator stays in the scratch.  It must not lie where a later call with more rows keeps the words
