@@ -132,7 +132,7 @@ struct DecodeBars {
   uint64_t red;  // cluster kernel: the other CTAs' partials of this CTA's rows have landed (counted in bytes)
   float    amax[4][64];
   float    inv[64];
-  float    row_max[2][4];  // reduction warps
+  float    row_max[2][4];  // reduction warps: maxima of the row they share, one set per group of the CTA
 };
 static_assert(sizeof(DecodeBars) <= 1536, "DecodeBars outgrew its slot in shared memory");
 
@@ -407,80 +407,80 @@ __device__ __forceinline__ bool reduce_split_groups(const SplitGroup (&g)[NG],
 }
 
 // The same for ONE group with many contributors (a left-over group of a shape with at least as many groups as CTAs is cut
-// into pieces of one or two K-blocks) and few rows: contributor j's four reduction warps take rows j, j + cnt, ...
+// into pieces of one or two K-blocks) and no more rows than those: contributor j's four reduction warps take row j
 // together, 32 columns each, one word per lane and contributor, so that CB contributors are in flight in CB registers.
 // With a warp per row (four words per lane, eight contributors in flight) the rows were finished two loaded L2 round
 // trips later, and the launch with them (19456x2560 at M = 1 / 16: 11.6 / 12.2 us, now 10.6 / 11.1 us).
+// `row_max` belongs to this call alone: a CTA that finishes a row in both of its groups gives each its own (nothing but
+// the one barrier below keeps the four warps together).
 template<int MP, bool OUT_F32, int CB>
-__device__ __forceinline__ void reduce_split_group_rows(const SplitGroup& g, int j0, int rw, float (&row_max)[2][4],
-                                                        uint32_t* __restrict__ partials, void* __restrict__ C_out, float* __restrict__ C_s,
-                                                        int M, int N, int lane, volatile uint32_t* abort_flag, uint32_t* status)
+__device__ __forceinline__ void reduce_split_group_row(const SplitGroup& g, int m, int rw, float (&row_max)[4],
+                                                       uint32_t* __restrict__ partials, void* __restrict__ C_out, float* __restrict__ C_s,
+                                                       int M, int N, int lane, volatile uint32_t* abort_flag, uint32_t* status)
 {
-  const int n = rw * 32 + lane;  // column inside the group
-  for (int m = j0, turn = 0; m < M; m += g.cnt, turn ^= 1) {
-    float sum = 0.0f;
-    for (int base = 0; base < g.cnt; base += CB) {
-      uint32_t*          src = partials + ((size_t)((g.c_lo + base) * 2) * MP + m) * 128 + n;
-      uint32_t           w[CB];
-      unsigned long long t0    = 0;
-      uint32_t           spins = 0;
-      for (;;) {
-        bool landed = true;
+  const int n   = rw * 32 + lane;  // column inside the group
+  float     sum = 0.0f;
+  for (int base = 0; base < g.cnt; base += CB) {
+    uint32_t*          src = partials + ((size_t)((g.c_lo + base) * 2) * MP + m) * 128 + n;
+    uint32_t           w[CB];
+    unsigned long long t0    = 0;
+    uint32_t           spins = 0;
+    for (;;) {
+      bool landed = true;
 #pragma unroll
-        for (int j = 0; j < CB; ++j) {
-          w[j] = 1u;
-          if (base + j < g.cnt) {
-            // (the group's first contributor reached it at K-block 0: slot 1)
-            asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(w[j]) : "l"(src + (j * 2 + (base + j == 0 ? 1 : 0)) * (MP * 128)) : "memory");
-          }
+      for (int j = 0; j < CB; ++j) {
+        w[j] = 1u;
+        if (base + j < g.cnt) {
+          // (the group's first contributor reached it at K-block 0: slot 1)
+          asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(w[j]) : "l"(src + (j * 2 + (base + j == 0 ? 1 : 0)) * (MP * 128)) : "memory");
         }
+      }
 #pragma unroll
-        for (int j = 0; j < CB; ++j) {
-          landed = landed && w[j] != 0u;
+      for (int j = 0; j < CB; ++j) {
+        landed = landed && w[j] != 0u;
+      }
+      if (__all_sync(0xffffffffu, landed)) {
+        break;
+      }
+      if ((++spins & 0x7) == 0) {
+        if (*abort_flag) {
+          break;  // (not a return: the four warps meet at a barrier below)
         }
-        if (__all_sync(0xffffffffu, landed)) {
+        const unsigned long long now = global_timer_ns();
+        if (t0 == 0) {
+          t0 = now;
+        }
+        else if (now - t0 > WAIT_LIMIT_NS) {
+          *abort_flag = DEV_WAIT_SPLITK;
+          atomicCAS(status, 0u, (uint32_t)DEV_WAIT_SPLITK);
           break;
         }
-        if ((++spins & 0x7) == 0) {
-          if (*abort_flag) {
-            break;  // (not a return: the four warps meet at a barrier below)
-          }
-          const unsigned long long now = global_timer_ns();
-          if (t0 == 0) {
-            t0 = now;
-          }
-          else if (now - t0 > WAIT_LIMIT_NS) {
-            *abort_flag = DEV_WAIT_SPLITK;
-            atomicCAS(status, 0u, (uint32_t)DEV_WAIT_SPLITK);
-            break;
-          }
-        }
       }
+    }
 #pragma unroll
-      for (int j = 0; j < CB; ++j) {  // ascending CTA order: the result does not depend on timing
-        if (base + j < g.cnt) {
-          __stcg(src + (j * 2 + (base + j == 0 ? 1 : 0)) * (MP * 128), 0u);  // consumed: back to zero for the next launch
-          sum += decode_partial(w[j]);
-        }
+    for (int j = 0; j < CB; ++j) {  // ascending CTA order: the result does not depend on timing
+      if (base + j < g.cnt) {
+        __stcg(src + (j * 2 + (base + j == 0 ? 1 : 0)) * (MP * 128), 0u);  // consumed: back to zero for the next launch
+        sum += decode_partial(w[j]);
       }
     }
-    if constexpr (OUT_F32) {
-      reinterpret_cast<float*>(C_out)[(size_t)m * N + (size_t)g.nb * 128 + n] = sum;
+  }
+  if constexpr (OUT_F32) {
+    reinterpret_cast<float*>(C_out)[(size_t)m * N + (size_t)g.nb * 128 + n] = sum;
+  }
+  else {
+    // largest magnitude of the row, NaN passed over unless there is nothing else (as fmaxf does)
+    const float a  = fabsf(sum);
+    const int   mx = __reduce_max_sync(0xffffffffu, a == a ? __float_as_int(a) : -1);
+    if (lane == 0) {
+      row_max[rw] = __int_as_float(mx);
     }
-    else {
-      // largest magnitude of the row, NaN passed over unless there is nothing else (as fmaxf does)
-      const float a  = fabsf(sum);
-      const int   mx = __reduce_max_sync(0xffffffffu, a == a ? __float_as_int(a) : -1);
-      if (lane == 0) {
-        row_max[turn][rw] = __int_as_float(mx);
-      }
-      asm volatile("bar.sync 2, 128;" ::: "memory");  // (alternating rows of row_max: one barrier per row)
-      const float amax = fmaxf(fmaxf(row_max[turn][0], row_max[turn][1]), fmaxf(row_max[turn][2], row_max[turn][3]));
-      const float inv  = amax > 0.0f ? __fdiv_rn(448.0f, amax) : 0.0f;
-      reinterpret_cast<uint8_t*>(C_out)[(size_t)m * N + (size_t)g.nb * 128 + n] = (uint8_t)__nv_cvt_float_to_fp8(sum * inv, __NV_SATFINITE, __NV_E4M3);
-      if (n == 0) {
-        C_s[(size_t)g.nb * M + m] = __fdiv_rn(amax, 448.0f);
-      }
+    asm volatile("bar.sync 2, 128;" ::: "memory");
+    const float amax = fmaxf(fmaxf(row_max[0], row_max[1]), fmaxf(row_max[2], row_max[3]));
+    const float inv  = amax > 0.0f ? __fdiv_rn(448.0f, amax) : 0.0f;
+    reinterpret_cast<uint8_t*>(C_out)[(size_t)m * N + (size_t)g.nb * 128 + n] = (uint8_t)__nv_cvt_float_to_fp8(sum * inv, __NV_SATFINITE, __NV_E4M3);
+    if (n == 0) {
+      C_s[(size_t)g.nb * M + m] = __fdiv_rn(amax, 448.0f);
     }
   }
 }
@@ -1034,15 +1034,15 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
         if constexpr (MP <= 16) {
           // Groups with many contributors: a row per CTA and its four warps.  (The choice is a property of the group: every
           // contributor makes the same one.)  A warp per row takes eight contributors at a time, so it is as good up to
-          // eight, and up to sixteen where the four warps would have more than one row to do.
+          // eight, and where the four warps would have more than one row to do.
           max_cnt = 0;
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
-            if (k < n_pend && g[k].cnt > (M <= g[k].cnt ? 8 : 16)) {
-              const int j0 = (int)blockIdx.x - g[k].c_lo;
-              if (j0 < M) {
-                wait_contributors<MP>(g[k], partials, j0, rw * 32, lane, abort_flag, status);
-                reduce_split_group_rows<MP, OUT_F32, 24>(g[k], j0, rw, bars->row_max, partials, C_out, C_s, M, N, lane, abort_flag, status);
+            if (k < n_pend && g[k].cnt > 8 && M <= g[k].cnt) {
+              const int m = (int)blockIdx.x - g[k].c_lo;
+              if (m < M) {
+                wait_contributors<MP>(g[k], partials, m, rw * 32, lane, abort_flag, status);
+                reduce_split_group_row<MP, OUT_F32, 24>(g[k], m, rw, bars->row_max[k], partials, C_out, C_s, M, N, lane, abort_flag, status);
               }
               g[k].mine = false;
             }

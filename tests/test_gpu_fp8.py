@@ -116,6 +116,40 @@ def test_left_over_groups_with_many_contributors(capi, oracle, cuda, M, NK):
     assert np.array_equal(gq, gq2) and np.array_equal(gs, gs2) and np.array_equal(gf, gf2)
 
 
+def ctas_with_a_row_in_two_groups(M, N, K, ctas=148):
+    """CTAs of the stream-K decode kernel that finish a row in both of their cut groups with four warps to the row (more than
+    eight contributors, no more rows than those), from the split rule: the left-over groups cut evenly among the CTAs."""
+    groups, kb = N // 128, K // 128
+    tail = (groups - groups // ctas * ctas) * kb
+    n = min(tail, ctas)
+    runs = [(c * tail // n, (c + 1) * tail // n) for c in range(n)]
+    found = []
+    for c, (lo, hi) in enumerate(runs):
+        rows = 0
+        for g in {lo // kb, (hi - 1) // kb}:
+            part = [i for i, (a, b) in enumerate(runs) if a < (g + 1) * kb and b > g * kb]
+            rows += len(part) > 8 and M <= len(part) and c - part[0] < M
+        if rows == 2:
+            found.append(c)
+    return found
+
+
+@pytest.mark.parametrize("shape", [(15, 1280, 4096), (15, 1280, 2560), (16, 1280, 9728), (13, 20480, 2560), (11, 20736, 2560), (14, 20352, 4096)])
+def test_one_cta_finishes_a_row_in_two_groups(capi, oracle, cuda, shape):
+    # the two rows follow one another in the same four warps: each has its own exchange of row maxima
+    M, N, K = shape
+    assert ctas_with_a_row_in_two_groups(M, N, K)
+    case = make_case(oracle, 49, M, N, K)
+    gq, gs, gf = gpu_mm(capi, cuda, *case)
+    assert "stream-K" in capi.describe_plan("fp8", M, N, K)
+    check_against_oracle(oracle, *case, gq, gs, gf)
+    dev = to_dev(cuda, *case)
+    Cq, Cs = torch.empty((M, N), dtype=torch.uint8, device=cuda), torch.empty((N // 128, M), device=cuda)
+    for _ in range(50):
+        capi.fp8_blockwise_mm(*dev, Cq, Cs, M, N, K)
+        assert np.array_equal(Cq.cpu().numpy(), gq) and np.array_equal(Cs.cpu().numpy(), gs)
+
+
 @pytest.mark.parametrize("M", [1, 16, 64])
 @pytest.mark.parametrize("NK", QWEN3_4B)
 def test_qwen3_4b_decode_shapes(capi, oracle, cuda, M, NK):
