@@ -28,7 +28,8 @@ __device__ __forceinline__ void store_group_row(float4 s, int m, int nb, void* _
 }
 
 // Several such rows of one warp at once: lane j does the two divisions of row j for everybody (one after the other
-// they took half of the time).  Rows whose group is not below n_groups are left out.
+// they took half of the time).  Rows whose group is not below n_groups are left out.  The maximum starts from zero and
+// passes NaN over, as in the kernels whose threads hold whole rows: the finite values of a group keep their scale and codes.
 template<bool OUT_F32, int ROWS>
 __device__ __forceinline__ void store_group_rows(const float4 (&s)[ROWS], const int (&m)[ROWS], const int (&nb)[ROWS], int n_groups,
                                                  void* __restrict__ C_out, float* __restrict__ C_s, int M, int N, int lane)
@@ -46,7 +47,7 @@ __device__ __forceinline__ void store_group_rows(const float4 (&s)[ROWS], const 
     int   row   = 0, group = n_groups;
 #pragma unroll
     for (int j = 0; j < ROWS; ++j) {
-      const float mine = fmaxf(fmaxf(fabsf(s[j].x), fabsf(s[j].y)), fmaxf(fabsf(s[j].z), fabsf(s[j].w)));
+      const float mine = fmaxf(fmaxf(fmaxf(0.0f, fabsf(s[j].x)), fabsf(s[j].y)), fmaxf(fmaxf(0.0f, fabsf(s[j].z)), fabsf(s[j].w)));
       const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mine)));
       if (lane == j) {
         amax  = most;

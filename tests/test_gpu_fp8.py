@@ -292,6 +292,38 @@ def test_pair_kernel_128_row_tiles(capi, oracle, cuda, shape):
     assert np.array_equal(gq2, gq3) and np.array_equal(gs2, gs3) and np.array_equal(gf2, gf3)
 
 
+@pytest.mark.parametrize("shape", [(100, 512, 2176), (100, 9472, 256), (300, 384, 1664), (700, 2560, 512)])
+@pytest.mark.parametrize("gather", [False, True])
+def test_nan_columns_leave_the_rest_of_their_group_alone(capi, oracle, cuda, shape, gather):
+    # Four adjacent weight rows of NaN codes (the four columns of one lane) and one activation row of them, on tiles that
+    # are cut along K and on whole ones: every other code and scale is what it is with those weight rows zero.
+    M, N, K = shape
+    A_q, A_s, B_q, B_s = make_case(oracle, 50, M, N, K)
+    bad = slice(N - 128 + 60, N - 128 + 64)
+    A_q[M - 3] = 0x7F
+    dA, dAs, dB, dBs = to_dev(cuda, A_q, A_s, B_q, B_s)
+    capi.ensure_workspace(M, N, K)
+    assert "pair_kernel_m128" in capi.describe_plan("fp8", M, N, K)
+    outs = []
+    for code in (0x00, 0x7F):
+        dB[bad] = code
+        Cq, Cs = torch.full((M, N), 0xAA, dtype=torch.uint8, device=cuda), torch.full((N // 128, M), -1.0, device=cuda)
+        if gather:
+            capi.fp8_blockwise_mm_gather(dA, dAs, dB, dBs, [Cq], [Cs], N, 0, M, N, K)
+        else:
+            capi.fp8_blockwise_mm(dA, dAs, dB, dBs, Cq, Cs, M, N, K)
+        torch.cuda.synchronize()
+        outs.append((Cq.cpu().numpy(), Cs.cpu().numpy()))
+    capi.check_status()
+    (q0, s0), (q1, s1) = outs
+    assert np.isfinite(s1).all() and np.array_equal(s0, s1)
+    assert (s1[:, M - 3] == 0).all() and ((q1[M - 3] & 0x7F) == 0x7F).all()
+    assert ((q1[:, bad] & 0x7F) == 0x7F).all()
+    other = np.ones(N, dtype=bool)
+    other[bad] = False
+    assert np.array_equal(q0[:, other], q1[:, other])
+
+
 def gpu_c_quant(acc):
     """The output quantisation rule in torch fp32 on the GPU (for full-size property checks)."""
     M, N = acc.shape

@@ -140,6 +140,20 @@ def test_swiglu_128_row_tiles(capi, oracle, cuda, shape):
     assert np.array_equal(gq, gq2) and np.array_equal(gs, gs2)
 
 
+def test_nan_columns_leave_the_rest_of_their_group_alone(capi, oracle, cuda):
+    # (the four columns of one lane of the 128-row kernel's row-wise finish; a zero gate gives a zero)
+    M, I, K = 65, 1152, 384
+    case = make_case(oracle, 99, M, I, K)
+    outs = []
+    for code in (0x00, 0x7F):
+        case[2][64:68] = code
+        outs.append(run(capi, cuda, case, M, I, K))
+    (q0, s0), (q1, s1) = outs
+    assert np.isfinite(s1).all() and np.array_equal(s0, s1)
+    assert ((q1[:, 64:68] & 0x7F) == 0x7F).all()
+    assert np.array_equal(q0[:, :64], q1[:, :64]) and np.array_equal(q0[:, 68:], q1[:, 68:])
+
+
 @pytest.mark.parametrize("M", [33, 64])
 def test_decode_call_after_a_hook_call_with_fewer_rows(capi, oracle, cuda, M):
     # The hook's accumulator stays in the scratch.  It must not lie where a later call with more rows keeps the words
