@@ -143,12 +143,10 @@ size_t llmmm_fp8_swiglu_workspace_bytes(int M, int I, int K);
  *   positions [M] int32 (rows of the angle tables), cos_table / sin_table [table_rows, 64] fp32, weights [128] fp32.
  *   A position outside [0, table_rows) is clamped to the nearest row (no access outside the tables is made) and
  *   recorded: llmmm_check_status then returns LLMMM_ERR_DEVICE_WAIT with code 0x201.
- * Requires K%128 == 0, any M >= 1; tables, weights, A, B_t and C 16-byte aligned.  M > 128 runs one fused kernel
+ * Requires K%128 == 0, any M >= 1; tables, weights, A, B_t and C 16-byte aligned.  M > 64 runs one fused kernel
  * (256-row tiles, always whole: registered scratch is not used).  M <= 64 runs the
  * weight-streaming decode kernel into scratch followed by a small kernel, provided the registered scratch has
- * llmmm_fp8_qk_norm_rope_workspace_bytes(M, N, K) bytes; so does M <= 128 with the 128-row kernel where the plain GEMM
- * runs on that and the registered scratch has room for the [M, N] accumulator; otherwise the 256-row kernel runs for
- * small M too. */
+ * llmmm_fp8_qk_norm_rope_workspace_bytes(M, N, K) bytes; otherwise the 256-row kernel runs for small M too. */
 int llmmm_fp8_blockwise_mm_qk_norm_rope_e4m3out(const void*    A,
                                                 const float*   A_scale_t,
                                                 const void*    B_t,

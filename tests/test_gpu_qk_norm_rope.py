@@ -151,14 +151,19 @@ def test_decode_sized(capi, oracle, cuda, M):
 @pytest.mark.parametrize("M", [65, 128])
 @pytest.mark.parametrize("weights", [True, False])
 def test_65_to_128_rows(capi, oracle, cuda, M, weights):
-    # with scratch: the 128-row pair kernel + the small hook kernel; without, the fused 256-row kernel
+    # One fused kernel that leaves the registered scratch alone: a GEMM on another stream may be using it.
     c = make_case(oracle, 75, M, 16, 4, 1152, weights=weights)
     capi.clear_workspace()
     gq, gs = run(capi, cuda, c)
     check(oracle, c, gq, gs)
     capi.ensure_workspace(c["M"], c["N"], c["K"])
-    gq2, gs2 = run(capi, cuda, c, launches=2)
-    check(oracle, c, gq2, gs2)
+    capi.ensure_workspace_bytes(capi.fp8_workspace_bytes(64, c["N"], c["K"]) + 4 * M * c["N"])
+    ws = capi._workspaces[torch.cuda.current_device()]
+    assert "pair_kernel_m128" in capi.describe_plan("fp8_f32out", c["M"], c["N"], c["K"])
+    before = ws.clone()
+    gq2, gs2 = run(capi, cuda, c)
+    assert torch.equal(ws, before)
+    assert (gq2 == gq).all() and (gs2 == gs).all()
 
 
 def test_argument_errors(capi, cuda):
