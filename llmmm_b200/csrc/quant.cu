@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(256)
 // quantisation of y.  One CTA per row: it sums the squares, then scales and quantises one 128-wide group per
 // warp at a time.  A row of up to 8192 values is kept in registers in between (one pass over memory); a longer
 // one is re-read from L2.
+constexpr int RN_SUM_THREADS = 256;  // threads that add up the squares
 
 // RESIDENT: float4 values of the row a thread keeps (0: none, the row is re-read from L2 for the second phase).
 template<int RN_THREADS, int RESIDENT>
@@ -164,7 +165,8 @@ __global__ void __launch_bounds__(RN_THREADS)
   rmsnorm_quant_1x128_kernel(const float* __restrict__ x, const float* __restrict__ weight, float eps, uint8_t* __restrict__ q,
                              float* __restrict__ scale, int M, int K)
 {
-  __shared__ float warp_sum[RN_THREADS / 32];
+  static_assert(RN_THREADS == RN_SUM_THREADS || (RN_THREADS == 2 * RN_SUM_THREADS && RESIDENT > 0), "order of the sum of squares");
+  __shared__ float warp_sum[RN_SUM_THREADS / 32];
   pdl_launch_dependents();
   pdl_wait();
   const int     lane = threadIdx.x & 31;
@@ -183,12 +185,38 @@ __global__ void __launch_bounds__(RN_THREADS)
       const int i = threadIdx.x + j * RN_THREADS;
       v[j]        = i < K / 4 ? __ldg(row + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
+    // Whatever M and K are, the squares are added in the order of 256 threads: thread t takes float4 t, t + 256, ... of the
+    // row (zeros beyond its end add nothing), so that a row's result does not depend on how many rows there are.  With
+    // 512 threads the upper half hands its values over (1 x 2560: 2.19 us, 2.17 if all
+    // 512 add; 100 x 4096 2.67 and 2.66).
+    auto add = [&](const float4& t) {
+      ss = fmaf(t.x, t.x, ss);
+      ss = fmaf(t.y, t.y, ss);
+      ss = fmaf(t.z, t.z, ss);
+      ss = fmaf(t.w, t.w, ss);
+    };
+    if constexpr (RN_THREADS == 2 * RN_SUM_THREADS) {
+      __shared__ float4 upper[RESIDENT][RN_SUM_THREADS];
+      if (threadIdx.x >= RN_SUM_THREADS) {
 #pragma unroll
-    for (int j = 0; j < RESIDENT; ++j) {  // (zeros beyond the row add nothing: same sum, same order as below)
-      ss = fmaf(v[j].x, v[j].x, ss);
-      ss = fmaf(v[j].y, v[j].y, ss);
-      ss = fmaf(v[j].z, v[j].z, ss);
-      ss = fmaf(v[j].w, v[j].w, ss);
+        for (int j = 0; j < RESIDENT; ++j) {
+          upper[j][threadIdx.x - RN_SUM_THREADS] = v[j];
+        }
+      }
+      __syncthreads();
+      if (threadIdx.x < RN_SUM_THREADS) {
+#pragma unroll
+        for (int j = 0; j < RESIDENT; ++j) {
+          add(v[j]);
+          add(upper[j][threadIdx.x]);
+        }
+      }
+    }
+    else {
+#pragma unroll
+      for (int j = 0; j < RESIDENT; ++j) {
+        add(v[j]);
+      }
     }
   }
   else {
@@ -204,13 +232,13 @@ __global__ void __launch_bounds__(RN_THREADS)
   for (int o = 16; o > 0; o >>= 1) {
     ss += __shfl_xor_sync(0xffffffffu, ss, o);
   }
-  if (lane == 0) {
+  if (lane == 0 && warp < RN_SUM_THREADS / 32) {
     warp_sum[warp] = ss;
   }
   __syncthreads();
   float total = 0.0f;
 #pragma unroll
-  for (int i = 0; i < RN_THREADS / 32; ++i) {
+  for (int i = 0; i < RN_SUM_THREADS / 32; ++i) {
     total += warp_sum[i];  // the same order in every thread
   }
   const float inv = __frsqrt_rn(__fdiv_rn(total, (float)K) + eps);
@@ -391,9 +419,7 @@ int llmmm_fp8_rmsnorm_quant_1x128(const float* x, const float* weight, float eps
                       static_cast<uint8_t*>(q), scale, M, K);
   };
   // Up to a row per SM a row is a latency: as many threads as share it well (M = 1, K = 2560: 512 threads 2.3 us, 256 2.6, 128
-  // 3.2).  More rows: as few resident values as the row needs, registers decide how many rows an SM works on at a time;
-  // short rows in large numbers run best with more, smaller CTAs (4096 x 2560: 128 threads 13.4 us, 256 14.6; 1333 x 2560:
-  // 5.9 and 5.4; 8192 x 3584: 30.2 and 31.5 us).
+  // 3.2).  More rows: as few resident values as the row needs, registers decide how many rows an SM works on at a time.
   const bool few = M <= device->sm_count;
   LLMMM_CUDA_TRY(K > 8192        ? launch(rmsnorm_quant_1x128_kernel<256, 0>, 256)
                  : few && K > 4096 ? launch(rmsnorm_quant_1x128_kernel<512, 4>, 512)
@@ -401,7 +427,6 @@ int llmmm_fp8_rmsnorm_quant_1x128(const float* x, const float* weight, float eps
                  : few             ? launch(rmsnorm_quant_1x128_kernel<512, 1>, 512)
                  : K > 4096        ? launch(rmsnorm_quant_1x128_kernel<256, 8>, 256)
                  : K > 3072        ? launch(rmsnorm_quant_1x128_kernel<256, 4>, 256)
-                 : K > 2048 && K <= 2560 && M >= 2048 ? launch(rmsnorm_quant_1x128_kernel<128, 5>, 128)
                  : K > 2048        ? launch(rmsnorm_quant_1x128_kernel<256, 3>, 256)
                                    : launch(rmsnorm_quant_1x128_kernel<256, 2>, 256));
   g_launches.fetch_add(1);

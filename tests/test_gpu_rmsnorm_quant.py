@@ -56,6 +56,26 @@ def test_rmsnorm_quant_against_oracle(capi, oracle, cuda, shape):
         assert (gq[3] == 0).all() and (gs[:, 3] == 0).all()
 
 
+@pytest.mark.parametrize("K", [128, 1280, 2048, 2176, 2560, 2688, 4096, 4224, 8192, 8320])
+def test_a_row_does_not_depend_on_the_number_of_rows(capi, cuda, K):
+    # every form of the kernel adds the squares in the same order
+    g = torch.Generator(device=cuda).manual_seed(102)
+    x = torch.randn(4096, K, device=cuda, generator=g)
+    w = torch.rand(K, device=cuda, generator=g) + 0.5
+
+    def rows(M):
+        q, s = torch.empty(M, K, dtype=torch.uint8, device=cuda), torch.empty(K // 128, M, device=cuda)
+        capi.fp8_rmsnorm_quant_1x128(x[:M], w, 1e-6, q, s, M, K)
+        return q, s
+
+    q, s = rows(300)
+    for M in (1, 16, 148, 149, 2047, 2048, 4096):
+        n = min(M, 300)
+        q2, s2 = rows(M)
+        assert torch.equal(q2[:n], q[:n]) and torch.equal(s2[:, :n], s[:, :n]), M
+    capi.check_status()
+
+
 def test_rmsnorm_quant_equals_norm_then_quant(capi, cuda):
     M, K = 4096, 2560
     g = torch.Generator(device=cuda).manual_seed(101)
