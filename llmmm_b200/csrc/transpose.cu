@@ -7,28 +7,27 @@
 // tiles inside one warp's registers; here a CTA stages a tile in shared memory:
 //   * 4-byte: 64x64-word tiles, 1-byte: 128x128-byte tiles; a thread transposes 4x4 blocks in registers
 //     (bytes by permutes), stored under an XOR swizzle that keeps both the transposed writes and the row
-//     reads free of bank conflicts; global memory sees 16-byte accesses only.
+//     reads free of bank conflicts; global memory sees 16-byte accesses only;
+//   * small 4-byte matrices: 32x32-word tiles, padded rows (33 words).
 #include "host_common.h"
 #include "sm100.cuh"
 
 namespace llmmm {
 
-// TILE x TILE words per CTA.  A thread transposes a 4x4-word block in registers, so that global and shared memory are only
+// 64x64 words per CTA.  A thread transposes a 4x4-word block in registers, so that global and shared memory are only
 // touched with 16-byte accesses.  Output row c of the tile lies in T[c] with its 16-byte chunks XOR-swizzled by c / 4: the
 // eight lanes of a shared-memory phase write (eight column blocks, one row block) and read (eight chunks of one row)
-// eight different bank groups.  HBM-bound with tiles of 64: 6430 GB/s at 19456x2560, 62 us, where 32x32-word tiles moved
-// with 4-byte accesses took 87 us (tiles of 128x64, 64x128 and 32x128 words: 62 to 65 us).
-template<int TILE>
-__global__ void __launch_bounds__(TILE * TILE / 16) transpose_b32_kernel(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, int M, int N)
+// eight different bank groups.  HBM-bound: 6430 GB/s at 19456x2560, 62 us, where the kernel below takes 77 to 87 us
+// (tiles of 128x64, 64x128 and 32x128 words: 62 to 65 us).
+__global__ void __launch_bounds__(256) transpose_b32_kernel(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, int M, int N)
 {
-  constexpr int    B = TILE / 4;  // 4x4-word blocks along an edge
-  __shared__ uint4 T[TILE][B];
+  __shared__ uint4 T[64][16];
   pdl_launch_dependents();  // see sm100.cuh: the next kernel may start its set-up, this one waits for its predecessor
   pdl_wait();
-  const int tx = threadIdx.x % B;  // 4-column block of the input tile
-  const int ry = threadIdx.x / B;  // 4-row block
-  const int m0 = blockIdx.y * TILE;
-  const int n0 = blockIdx.x * TILE;
+  const int tx = threadIdx.x % 16;  // 4-column block of the input tile
+  const int ry = threadIdx.x / 16;  // 4-row block
+  const int m0 = blockIdx.y * 64;
+  const int n0 = blockIdx.x * 64;
   uint4     v[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -41,8 +40,32 @@ __global__ void __launch_bounds__(TILE * TILE / 16) transpose_b32_kernel(uint32_
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const int c = ry + B * j;  // output row inside the tile = input column; this thread's chunk of it: tx
+    const int c = ry + 16 * j;  // output row inside the tile = input column; this thread's chunk of it: tx
     __stcs(reinterpret_cast<uint4*>(dst + (size_t)(n0 + c) * M + m0) + tx, T[c][tx ^ (c >> 2)]);
+  }
+}
+
+// 32x32 words per CTA, one word per access: few words per thread and eight warps per tile, for matrices that do not fill
+// the GPU several times over.
+__global__ void __launch_bounds__(256) transpose_b32_small_kernel(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, int M, int N)
+{
+  __shared__ uint32_t tile[32][33];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tx = threadIdx.x & 31;
+  const int ty = threadIdx.x >> 5;
+  const int m0 = blockIdx.y * 32;
+  const int n0 = blockIdx.x * 32;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int r = ty + 8 * j;
+    tile[r][tx] = __ldcs(src + (size_t)(m0 + r) * N + n0 + tx);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int r = ty + 8 * j;  // output row inside the tile = input column
+    __stcs(dst + (size_t)(n0 + r) * M + m0 + tx, tile[tx][r]);
   }
 }
 
@@ -114,15 +137,16 @@ extern "C" int llmmm_transpose_aligned_128(void* dst, const void* src, int M, in
   }
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (elem_bytes == 4) {
-    // tiles of 64 need a few CTAs per SM to cover the latency of their loads (1024x1024, 256 tiles: 2.7 us against 2.2 us with
-    // tiles of 32)
+    // Up to about five 64x64-word tiles per SM the small kernel is the faster one (1024x1024: 2.04 against 2.91 us, 2048x1024
+    // 3.60 / 4.24, 2560x1024 4.33 / 4.61; 1280x2560 4.89 / 4.83, 2048x2048 5.94 / 5.43).  Its tiles with 16-byte accesses by
+    // 64 threads: 2.65 us at 1024x1024, 4.24 at 2048x1024.
     uint32_t*       d = static_cast<uint32_t*>(dst);
     const uint32_t* w = static_cast<const uint32_t*>(src);
-    if ((long long)(N / 64) * (M / 64) >= 4 * device->sm_count) {
-      LLMMM_CUDA_TRY(launch_pdl(transpose_b32_kernel<64>, dim3(N / 64, M / 64), dim3(256), 0, s, 1, d, w, M, N));
+    if ((long long)(N / 64) * (M / 64) >= 5 * device->sm_count) {
+      LLMMM_CUDA_TRY(launch_pdl(transpose_b32_kernel, dim3(N / 64, M / 64), dim3(256), 0, s, 1, d, w, M, N));
     }
     else {
-      LLMMM_CUDA_TRY(launch_pdl(transpose_b32_kernel<32>, dim3(N / 32, M / 32), dim3(64), 0, s, 1, d, w, M, N));
+      LLMMM_CUDA_TRY(launch_pdl(transpose_b32_small_kernel, dim3(N / 32, M / 32), dim3(256), 0, s, 1, d, w, M, N));
     }
   }
   else {

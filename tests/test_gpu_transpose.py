@@ -6,7 +6,8 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(128, 128), (256, 384), (4096, 4096), (6144, 2048), (2048, 12288)]
+SHAPES = [(128, 128), (256, 384), (4096, 4096), (6144, 2048), (2048, 12288),
+          (23552, 128), (128, 23680), (1024, 3072)]  # both sides of the choice between tiles of 32 and 64 words
 
 
 @pytest.mark.parametrize("shape", SHAPES)
