@@ -1,4 +1,5 @@
-"""Builds libllmmm_b200.so (the C-ABI library) in-tree with nvcc for sm_100a, and _binding.so (its calls for Python).
+"""Builds libllmmm_b200.so (the C-ABI library) in-tree with nvcc for sm_100a and, where torch is installed, _binding.so
+(its calls for Python).
 
 Usage: python -m llmmm_b200.build [--force] [--verbose] [--profile]
 
@@ -10,6 +11,7 @@ call the dump function).  The regular library contains none of this.
 from __future__ import annotations
 
 import concurrent.futures as cf
+import importlib.util
 import os
 import subprocess
 import sys
@@ -89,19 +91,26 @@ def build_library(force: bool = False, verbose: bool = False, profile: bool = Fa
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    if not profile:
+    if not profile and importlib.util.find_spec("torch") is not None:  # (a C or C++ host needs the library alone)
         build_binding(force)
     return lib
+
+
+def binding_built_for() -> str:
+    """What _binding.so is built against; capi.py does not use one that says otherwise."""
+    import torch
+    return f"torch {torch.__version__}, python {sys.version_info.major}.{sys.version_info.minor}"
 
 
 def build_binding(force: bool = False) -> Path:
     """_binding.so: the native form of the calls in capi.py, against the headers of the torch it will run with."""
     src = CSRC / "binding.cpp"
-    if not force and _newer(BINDING, [src, PKG.parent / "include" / "llmmm_c.h"]):
+    built_for = binding_built_for()
+    if not force and _newer(BINDING, [src, PKG.parent / "include" / "llmmm_c.h"]) and built_for.encode() + b"\0" in BINDING.read_bytes():
         return BINDING
     import torch
     root = Path(torch.__file__).resolve().parent
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f'-DLLMMM_BUILT_FOR="{built_for}"', f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            f"-I{root / 'include'}", f"-I{root / 'include/torch/csrc/api/include'}", f"-I{Path(NVCC).resolve().parent.parent / 'include'}",
            f"-I{sysconfig.get_paths()['include']}", str(src), "-o", str(BINDING), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch",
            "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-L{PKG}", f"-l:{LIB.name}", "-Wl,-rpath,$ORIGIN"]

@@ -10,19 +10,28 @@ torch is used only to hold device memory and to name the current stream.
 There is no fallback: if the shared library is missing, loading raises.
 
 The calls a token loop makes go through `_binding` (csrc/binding.cpp), which
-makes the same call of the same library in a fifth of the host time; what it
-does not take (it returns False) goes through ctypes below.
+makes the same call of the same library in a third of the host time (2.7-4.7 us
+against 9-12 us); what it does not take (it returns False) goes through ctypes
+below, and so does everything, after a warning, where it was not built for the
+torch in use.
 """
 from __future__ import annotations
 
 import ctypes
+import sys
+import warnings
 from pathlib import Path
 
 import torch
 
 try:
     from . import _binding as _native
-except ImportError:  # built against another torch, or not built: ctypes only
+    _built_for = getattr(_native, "BUILT_FOR", "another torch")
+    _native_missing = "" if _built_for == f"torch {torch.__version__}, python {sys.version_info.major}.{sys.version_info.minor}" \
+        else f"it was built for {_built_for}"
+except ImportError as e:
+    _native_missing = str(e)
+if _native_missing:
     _native = None
 
 _LIB_PATH = Path(__file__).resolve().parent / "libllmmm_b200.so"
@@ -39,6 +48,9 @@ def lib() -> ctypes.CDLL:
         if not _LIB_PATH.exists():
             raise RuntimeError(
                 f"{_LIB_PATH} is missing: build it with `python -m llmmm_b200.build`; there is no fallback path")
+        if _native is None:
+            warnings.warn(f"_binding.so is not used ({_native_missing}): calls cost the host about three times as much; build it with "
+                          "`python -m llmmm_b200.build`", stacklevel=2)
         L = ctypes.CDLL(str(_LIB_PATH))
         L.llmmm_last_error.restype = ctypes.c_char_p
         L.llmmm_version.restype = ctypes.c_char_p

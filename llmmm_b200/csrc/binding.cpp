@@ -220,5 +220,10 @@ PyModuleDef MODULE = {PyModuleDef_HEAD_INIT, "_binding", nullptr, -1, METHODS};
 
 PyMODINIT_FUNC PyInit__binding()
 {
-  return PyModule_Create(&MODULE);
+  PyObject* m = PyModule_Create(&MODULE);
+  if (m != nullptr && PyModule_AddStringConstant(m, "BUILT_FOR", LLMMM_BUILT_FOR) != 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
 }

@@ -3,6 +3,8 @@ header declares, validates arguments before touching a device, and refuses to
 compute without an sm_100 GPU (there is no CPU path to fall back to)."""
 import ctypes
 import re
+import subprocess
+import sys
 from pathlib import Path
 
 import pytest
@@ -103,3 +105,44 @@ def test_describe_plan_and_tune_validate_before_touching_a_device(capi):
     assert L.llmmm_describe_plan(capi.KINDS["fp8"], 4096, 4096, 4096, buf, n) == 2 and buf.value == b""
     assert L.llmmm_tune(capi.KINDS["bf16"], 4096, 4096) == 2
     assert L.llmmm_tune(9, 4096, 4096) == 2
+
+
+BUILD_SCRIPT = """
+import importlib.util, pathlib, sys
+{prelude}
+spec = importlib.util.spec_from_file_location("b", "llmmm_b200/build.py")
+b = importlib.util.module_from_spec(spec)
+spec.loader.exec_module(b)
+b.NVCC = "true"  # (everything is up to date: nothing is compiled or linked)
+{body}
+"""
+
+
+def build_script(prelude, body):
+    r = subprocess.run([sys.executable, "-c", BUILD_SCRIPT.format(prelude=prelude, body=body)], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return r.stdout
+
+
+def test_library_builds_without_torch(capi, tmp_path):
+    out = build_script("sys.modules['torch'] = None",
+                       f"b._newer = lambda target, deps: target.name != 'x.so'; b.BINDING = pathlib.Path({str(tmp_path)!r}) / 'x.so'\n"
+                       "print(b.build_library(), b.BINDING.exists())")
+    assert "libllmmm_b200.so False" in out
+
+
+def test_binding_of_another_torch_is_rebuilt_and_not_used(capi, tmp_path):
+    stale = tmp_path / "_binding.so"
+    stale.write_bytes(b"torch 0.0, python 3.0\0")
+    compiled = build_script("", f"b.BINDING = pathlib.Path({str(stale)!r}); ran = []\n"
+                            "class R: returncode = 0\n"
+                            "b.subprocess.run = lambda cmd, **kw: ran.append(cmd) or R\n"
+                            "b.build_binding(); print(len(ran))\n"
+                            "b.BINDING.write_bytes(b.binding_built_for().encode() + b'\\0'); ran.clear()\n"
+                            "b.build_binding(); print(len(ran))")
+    assert compiled.split() == ["1", "0"]
+    r = subprocess.run([sys.executable, "-W", "error", "-c",
+                        "import sys, types; m = types.ModuleType('llmmm_b200._binding'); m.BUILT_FOR = 'torch 0.0, python 3.0'\n"
+                        "sys.modules['llmmm_b200._binding'] = m\nfrom llmmm_b200 import capi\nassert capi._native is None\ncapi.lib()"],
+                       cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode != 0 and "_binding.so is not used (it was built for torch 0.0, python 3.0)" in r.stderr
