@@ -1251,7 +1251,7 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
 // For few rows, where tiles of 256 rows would be half empty or too few: here a pair shares a 128x256 tile
 // (tcgen05.mma.cta_group::2 with M = 128).  CTA r loads 64 rows of A_q and 128 of B_q (24 KB per K-block, seven stages: the weight stream from HBM is
 // the bound, 16 KB per SM every 364 ns).  Its 64 output rows lie in tensor memory twice: lanes 0-63 hold the tile's first
-// 128 columns, lanes 64-127 the second 128, so a partial is 128 columns wide and there are four partial stages.  Eight
+// 128 columns, lanes 64-127 the second 128, so a partial is 128 columns wide and there are four partial stages (three with FOLDS).  Eight
 // promotion warps: quarter q drains lanes 32 q .. (rows 32 (q & 1) .., scale group q / 2), and the two warps of a quarter
 // take 64 columns each; they meet at a 64-thread barrier for the row maxima.
 // With few tiles a tile is cut along K among the 2..4 pairs of a larger cluster, and their partial tiles are added through
@@ -1270,15 +1270,26 @@ constexpr int      BK         = 128;
 constexpr int      UMMA_K     = 32;
 constexpr uint32_t STAGES     = 7;
 constexpr int      THREADS    = 384;
-constexpr int      REGS_CTRL  = 56;
-constexpr int      REGS_PROMO = 224;
-static_assert(128 * REGS_CTRL + 256 * REGS_PROMO <= THREADS * 168, "setmaxnreg split exceeds the CTA's registers");
+// (a form with folds, see below, spilt in the control warps with 64)
+__host__ __device__ constexpr int regs_ctrl(bool folds) { return folds ? 72 : 56; }
+__host__ __device__ constexpr int regs_promo(bool folds) { return folds ? 216 : 224; }
+static_assert(128 * regs_ctrl(true) + 256 * regs_promo(true) <= THREADS * 168, "setmaxnreg split exceeds the CTA's registers");
+static_assert(128 * regs_ctrl(false) + 256 * regs_promo(false) <= THREADS * 168, "setmaxnreg split exceeds the CTA's registers");
 constexpr uint32_t A_BYTES    = 64 * BK;
 constexpr uint32_t B_BYTES    = 128 * BK;
 constexpr uint32_t STAGE_TX   = 2 * (A_BYTES + B_BYTES);
 constexpr int      SC_KB      = 4;   // ring of scale operands as in the 256-row kernel: 64 A scales and two B scales
 constexpr int      SC_SLOTS   = 4;
 constexpr int      SC_ROW     = 68;  // floats per K-block, padded to 16 bytes
+// FOLDS: every FOLD_KB K-blocks the running sum is added to a total in tensor memory, which takes the place of the fourth
+// partial stage.  For slices longer than those the 256-row kernel would cut (pair128_folds): one chain of 19 to 37 K-blocks
+// is further from the 64-bit sum than slices of 11 to 22 (fp32 output, 2-norm: 512x4096x4096 1.07e-7 against 0.84e-7; with
+// the total 0.84e-7; 100x2560x9728 9.5, 9.1 and 9.0e-8).  It costs 4 to 9 %, three stages and the folds about half each
+// (512x4096x4096 13.3 -> 14.1 us, 100x2560x9728 12.7 -> 13.4, 512x512x18944 17.0 -> 18.4; with the total in registers
+// twice that), which is why shorter slices run without.
+constexpr int      FOLD_KB    = 16;
+static_assert(FOLD_KB % SC_KB == 0, "folds lie between two slots of the scale ring");
+__host__ __device__ constexpr uint32_t parts(bool folds) { return folds ? 3 : 4; }
 constexpr uint32_t OFF_B      = STAGES * A_BYTES;
 constexpr uint32_t OFF_STG    = OFF_B + STAGES * B_BYTES;  // eight staging tiles of 4 KB (e4m3 output: 2 KB of them)
 constexpr uint32_t OFF_XCH    = OFF_STG + 8 * 4096;        // 256 floats: row maxima of the column halves
@@ -1304,7 +1315,7 @@ struct Fp8Pair128Bars {
 };
 static_assert(sizeof(Fp8Pair128Bars) <= 512, "barriers");
 
-template<int EPI>
+template<int EPI, bool FOLDS>
 __global__ void __launch_bounds__(fp8p128::THREADS, 1)
   fp8_blockwise_gemm_pair_kernel_m128(const __grid_constant__ CUtensorMap tm_a,
                                       const __grid_constant__ CUtensorMap tm_b,
@@ -1322,6 +1333,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
   using namespace fp8p128;
   constexpr bool OUT_F32 = EPI == EPI_F32, SWIGLU = EPI == EPI_SWIGLU;
   constexpr bool BY_ROW  = EPI != EPI_F32 && EPI != EPI_E4M3;  // rows are finished by warps even if the tile is not cut
+  constexpr uint32_t PARTS = parts(FOLDS);  // partial stages
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   Fp8Pair128Bars*    bars       = reinterpret_cast<Fp8Pair128Bars*>(smem + OFF_BAR);
@@ -1349,7 +1361,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
       mbar_init(&bars->full[s], 1);
       mbar_init(&bars->done[s], 1);
     }
-    for (int i = 0; i < 4; ++i) {
+    for (uint32_t i = 0; i < PARTS; ++i) {
       mbar_init(&bars->part_empty[i], 16);
     }
     for (int i = 0; i < SC_SLOTS; ++i) {
@@ -1378,7 +1390,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
   pdl_wait();
 
   if (warp < 4) {
-    setmaxnreg_dec<REGS_CTRL>();
+    setmaxnreg_dec<regs_ctrl(FOLDS)>();
     if (warp == 0) {
       // ---------------------------------------------------- TMA producer --
       if (lane == 0) {
@@ -1425,15 +1437,15 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
       const uint32_t     total = (uint32_t)(kb1 - kb0);
       for (uint32_t it = warp == 1 ? 0u : 1u; it < total; it += 2) {
         const uint32_t s = it % STAGES;
-        // (the stage's previous K-block is this thread's own: its phases are met in order)
-        mbar_wait(&bars->part_empty[it & 3], ((it >> 2) & 1) ^ 1, DEV_WAIT_TMEM_EMPTY, abort_flag, status);
+        const uint32_t p = it % PARTS;
+        mbar_wait(&bars->part_empty[p], ((it / PARTS) & 1) ^ 1, DEV_WAIT_TMEM_EMPTY, abort_flag, status);
         mbar_wait(&bars->full[s], (it / STAGES) & 1, DEV_WAIT_SMEM_FULL, abort_flag, status);
         tc_fence_after_sync();
         const uint64_t da = make_smem_desc_sw128(smem_u32(smem + s * A_BYTES), 0, 1024);
         const uint64_t db = make_smem_desc_sw128(smem_u32(smem + OFF_B + s * B_BYTES), 0, 1024);
 #pragma unroll
         for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-          tc_mma_f8_pair(tmem_base + (it & 3) * 128, da + (uint64_t)((kk * UMMA_K) >> 4), db + (uint64_t)((kk * UMMA_K) >> 4), idesc, kk != 0);
+          tc_mma_f8_pair(tmem_base + p * 128, da + (uint64_t)((kk * UMMA_K) >> 4), db + (uint64_t)((kk * UMMA_K) >> 4), idesc, kk != 0);
         }
         tc_commit_pair(&bars->done[s], (uint16_t)(3u << leader));
       }
@@ -1444,7 +1456,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
     }
   }
   else {
-    setmaxnreg_inc<REGS_PROMO>();
+    setmaxnreg_inc<regs_promo(FOLDS)>();
     // ------------------------------------------- promotion + epilogue ----
     const int      quarter      = warp & 3;         // tensor-memory lane quarter this warp may read
     const int      half         = (warp - 4) >> 2;  // which 64 columns of the scale group
@@ -1456,7 +1468,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
     const uint32_t sc_mine      = smem_u32(sc_ring) + ((quarter & 1) * 32 + lane) * 4;
     const uint32_t sc_b         = (64 - (quarter & 1) * 32 - lane + (quarter >> 1)) * 4;
     uint8_t*       stg          = smem + OFF_STG + (warp - 4) * 4096;
-    uint32_t       it = 0, st = 0, st_ph = 0, sc_slot = 0, sc_ph = 0;
+    uint32_t       it = 0, p3 = 0, st = 0, st_ph = 0, sc_slot = 0, sc_ph = 0;
     {
       const int  ng   = tile * 2 + (quarter >> 1);
       const bool m_ok = m < M;
@@ -1466,24 +1478,52 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
       for (int i = 0; i < 64; ++i) {
         acc[i] = 0.0f;
       }
+      // sum so far = total + acc, in tensor memory (columns of the fourth partial stage) or in acc
+      const uint32_t t_total = t_mine + PARTS * 128;
+      auto add_total = [&](int c) {
+        uint32_t t[32];
+        tmem_ld_32x32b_x32(t_total + c, t);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          acc[c + i] = __uint_as_float(t[i]) + acc[c + i];
+        }
+      };
       for (int left = kb1 - kb0; left > 0; left -= SC_KB) {
+        if (FOLDS && it != 0 && it % FOLD_KB == 0) {
+#pragma unroll
+          for (int c = 0; c < 64; c += 32) {
+            if (it != FOLD_KB) {
+              add_total(c);
+            }
+            uint32_t t[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              t[i]       = __float_as_uint(acc[c + i]);
+              acc[c + i] = 0.0f;
+            }
+            tmem_st_32x32b_x32(t_total + c, t);
+          }
+          tmem_st_wait();
+        }
         mbar_wait_at(bars_at + (uint32_t)offsetof(Fp8Pair128Bars, sc_full) + sc_slot * 8, sc_ph, DEV_WAIT_SMEM_FULL, abort_at, status);
         uint32_t       sc_addr = sc_mine + sc_slot * (SC_KB * SC_ROW * 4);
         const uint32_t sc_end  = sc_addr + min(left, SC_KB) * (SC_ROW * 4);
 #pragma unroll 1
         for (; sc_addr != sc_end; sc_addr += SC_ROW * 4) {
+          const uint32_t p = FOLDS ? p3 : it & 3;
           // one fp32 rounding of the scale product, as in the reference
           float sc = __fmul_rn(lds_f32(sc_addr), lds_f32(sc_addr + sc_b));
           mbar_wait_at(bars_at + (uint32_t)offsetof(Fp8Pair128Bars, done) + st * 8, st_ph, DEV_WAIT_TMEM_FULL, abort_at, status);
           tc_fence_after_sync();
           uint32_t v0[32], v1[32];
-          tmem_ld_32x32b_x32(t_mine + (it & 3) * 128, v0);
-          tmem_ld_32x32b_x32(t_mine + (it & 3) * 128 + 32, v1);
+          tmem_ld_32x32b_x32(t_mine + p * 128, v0);
+          tmem_ld_32x32b_x32(t_mine + p * 128 + 32, v1);
           tmem_ld_wait();
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) {
-            mbar_arrive_cluster_relaxed(empty_leader + (it & 3) * 8);
+            mbar_arrive_cluster_relaxed(empty_leader + p * 8);
           }
           asm volatile("" : "+f"(sc));  // the arithmetic stays behind the hand-back
 #pragma unroll
@@ -1495,6 +1535,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
             ffma2(acc[32 + i], acc[32 + i + 1], v1[i], v1[i + 1], sc);
           }
           ++it;
+          p3 = p3 == 2 ? 0 : p3 + 1;
           if (++st == STAGES) {
             st = 0;
             st_ph ^= 1;
@@ -1507,6 +1548,13 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
         if (++sc_slot == SC_SLOTS) {
           sc_slot = 0;
           sc_ph ^= 1;
+        }
+      }
+
+      if (FOLDS && it > FOLD_KB) {
+#pragma unroll
+        for (int c = 0; c < 64; c += 32) {
+          add_total(c);
         }
       }
 
@@ -1723,7 +1771,7 @@ static int pair128_capacity(const DeviceInfo* info, int ways)
   std::lock_guard<std::mutex> lock(mu);
   if (!known[info->device][ways]) {
     int clusters = 0;
-    if (cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_E4M3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES)
+    if (cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_E4M3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES)
         == cudaSuccess) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim            = dim3((unsigned)(2 * ways * (info->sm_count / (2 * ways))));
@@ -1736,7 +1784,7 @@ static int pair128_capacity(const DeviceInfo* info, int ways)
       attr[0].val.clusterDim.z = 1;
       cfg.attrs                = attr;
       cfg.numAttrs             = 1;
-      if (cudaOccupancyMaxActiveClusters(&clusters, fp8_blockwise_gemm_pair_kernel_m128<EPI_E4M3>, &cfg) != cudaSuccess) {
+      if (cudaOccupancyMaxActiveClusters(&clusters, fp8_blockwise_gemm_pair_kernel_m128<EPI_E4M3, false>, &cfg) != cudaSuccess) {
         clusters = 0;
       }
     }
@@ -1759,6 +1807,16 @@ static int pair128_ways(const DeviceInfo* info, int M, int N, int K)
     }
   }
   return 1;
+}
+
+// Whether a slice's sum is folded: where it is longer than the slices that the 256-row kernel would cut this problem into
+// (whole tiles there are one chain over K, longer than any slice here).
+static bool pair128_folds(const DeviceInfo* info, int M, int N, int K, int ways)
+{
+  const int       tiles256 = ((M + fp8pair::BM - 1) / fp8pair::BM) * ((N + fp8pair::BN - 1) / fp8pair::BN);
+  const int       k_blocks = K / fp8p128::BK, slice = (k_blocks + ways - 1) / ways;
+  const SplitPlan plan     = plan_split(info, tiles256, k_blocks, 4, 5, 3, false);
+  return slice > fp8p128::FOLD_KB && plan.split_pairs > 0 && slice > plan.split_chunk;
 }
 
 // Whether a problem that is the pair kernels' runs with 128-row tiles.  Up to 128 rows always.  Above, a 128-row tile has
@@ -1815,18 +1873,19 @@ static int launch_fp8_pair128(const void* A, const float* A_s, const void* B, co
                            EPI == EPI_F32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B))) {
     return LLMMM_ERR_CUDA;
   }
-  static thread_local bool attr_set[64] = {};
-  if (!attr_set[info->device]) {
-    LLMMM_CUDA_TRY(cudaFuncSetAttribute(
-      fp8_blockwise_gemm_pair_kernel_m128<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
-    attr_set[info->device] = true;
+  const int     ways   = EPI == EPI_SWIGLU ? 1 : pair128_ways(info, M, N, K);
+  const bool    folds  = EPI != EPI_SWIGLU && pair128_folds(info, M, N, K, ways);
+  auto* const   kernel = folds ? fp8_blockwise_gemm_pair_kernel_m128<EPI, EPI != EPI_SWIGLU> : fp8_blockwise_gemm_pair_kernel_m128<EPI, false>;
+  static thread_local bool attr_set[64][2] = {};
+  if (!attr_set[info->device][folds]) {
+    LLMMM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
+    attr_set[info->device][folds] = true;
   }
-  const int ways  = EPI == EPI_SWIGLU ? 1 : pair128_ways(info, M, N, K);
   const int tiles = ((M + BM - 1) / BM) * (EPI == EPI_SWIGLU ? N / 128 : (N + BN - 1) / BN);
   if (ways > 1) {
     g_split_launches.fetch_add(1);
   }
-  LLMMM_CUDA_TRY(launch_pdl(fp8_blockwise_gemm_pair_kernel_m128<EPI>, dim3((unsigned)(2 * ways * tiles)), dim3(THREADS), SMEM_BYTES,
+  LLMMM_CUDA_TRY(launch_pdl(kernel, dim3((unsigned)(2 * ways * tiles)), dim3(THREADS), SMEM_BYTES,
                             stream, (unsigned)(2 * ways), tm_a, tm_b, tm_c, A_s, B_s, C, C_s, M, N, K, gather, info->status));
   g_launches.fetch_add(1);
   return LLMMM_OK;
@@ -2021,10 +2080,13 @@ int warm_fp8_kernels(const DeviceInfo* info)
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_SWIGLU)));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_GATHER)));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_ROPE)));
-  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_E4M3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
-  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
-  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
-  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_E4M3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_E4M3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_F32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_F32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_SWIGLU, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_GATHER, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_GATHER, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8cfg::SMEM_BYTES));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8cfg::SMEM_BYTES));
   return warm_decode_kernels(info);

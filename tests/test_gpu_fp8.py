@@ -12,6 +12,7 @@ import numpy as np
 import pytest
 import torch
 
+from gpu_reference import fp8_blockwise_acc_f64
 from helpers import e4m3_ulp, fp8_sources
 
 pytestmark = pytest.mark.gpu
@@ -275,10 +276,10 @@ def test_mid_m_few_tiles_take_the_pair_kernel_with_scratch(capi, oracle, cuda, s
 
 
 @pytest.mark.parametrize("shape", [(1 + 64, 256, 1024), (127, 384, 2176), (128, 2560, 1280), (100, 6144, 1152), (65, 9472, 512),
-                                   (129, 2560, 2048), (191, 640, 3200), (257, 1280, 2560), (384, 896, 1152), (641, 512, 1280), (1030, 256, 4096)])
+                                   (129, 2560, 2048), (191, 640, 3200), (257, 1280, 2560), (384, 896, 1152), (641, 512, 1280), (1030, 256, 4096), (300, 512, 9344), (257, 1408, 9728), (65, 256, 16896)])
 def test_pair_kernel_128_row_tiles(capi, oracle, cuda, shape):
     # one to four pairs per tile (10 to 74 tiles), rows and column groups beyond the matrix, slices of K of unequal length,
-    # K-blocks that are no multiple of the scale ring's four
+    # K-blocks that are no multiple of the scale ring's four; slices with one and two folds of the sum
     M, N, K = shape
     case = make_case(oracle, 48, M, N, K)
     capi.clear_workspace()
@@ -290,6 +291,30 @@ def test_pair_kernel_128_row_tiles(capi, oracle, cuda, shape):
     assert np.abs(gf - gf2).max() <= 4e-6 * np.abs(gf).max()
     gq3, gs3, gf3 = gpu_mm(capi, cuda, *case)
     assert np.array_equal(gq2, gq3) and np.array_equal(gs2, gs3) and np.array_equal(gf2, gf3)
+
+
+@pytest.mark.parametrize("shape", [(512, 4096, 4096), (700, 2560, 4096)])
+def test_long_slices_are_folded(capi, cuda, shape):
+    # Whole tiles of 32 K-blocks, which the 256-row kernel would cut in two: their sums are kept in two pieces too.  Measured against the same rows of a larger problem, whose whole 256-row tiles are one chain over K: halves of a
+    # chain have 1 / sqrt(2) of its random-walk error (a quarter or so of it, the block sums, is common to both).
+    M, N, K = shape
+    big = 4096
+    A_q, A_s, B_q, B_s = full_size_case(capi, cuda, big, N, K, 63, 0.02)
+    capi.ensure_workspace(M, N, K)
+    assert "pair_kernel_m128" in capi.describe_plan("fp8_f32out", M, N, K)
+    C, C_big = torch.empty(M, N, device=cuda), torch.empty(big, N, device=cuda)
+    capi.fp8_blockwise_mm_f32(A_q[:M], A_s[:, :M].contiguous(), B_q, B_s, C, M, N, K)
+    out = [(torch.empty(M, N, dtype=torch.uint8, device=cuda), torch.empty(N // 128, M, device=cuda)) for _ in range(2)]
+    capi.fp8_blockwise_mm(A_q[:M], A_s[:, :M].contiguous(), B_q, B_s, *out[0], M, N, K)
+    capi.fp8_blockwise_mm_gather(A_q[:M], A_s[:, :M].contiguous(), B_q, B_s, [out[1][0]], [out[1][1]], N, 0, M, N, K)
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    capi.clear_workspace()
+    capi.fp8_blockwise_mm_f32(A_q, A_s, B_q, B_s, C_big, big, N, K)
+    torch.cuda.synchronize()
+    capi.check_status()
+    exact = fp8_blockwise_acc_f64(A_q[:M], A_s[:, :M], B_q, B_s)
+    err, err_big = (float((c.double() - exact).norm() / exact.norm()) for c in (C, C_big[:M]))
+    assert err <= 0.9 * err_big, (err, err_big)
 
 
 @pytest.mark.parametrize("shape", [(100, 512, 2176), (100, 9472, 256), (300, 384, 1664), (700, 2560, 512)])
