@@ -117,8 +117,7 @@ __global__ void __launch_bounds__(256)
   quant_128x128_kernel(const float* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale, int rows, int cols)
 {
   __shared__ float warp_amax[8];
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait();  // (no pdl_launch_dependents(): this kernel writes weights, see sm100.cuh)
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int cb   = blockIdx.x;

@@ -202,8 +202,15 @@ __device__ __forceinline__ void mbar_wait_at(uint32_t bar_addr, uint32_t parity,
 // A kernel launched with cudaLaunchAttributeProgrammaticStreamSerialization may start while its
 // predecessor on the stream is still running; pdl_wait() then blocks until that predecessor has
 // completed and its memory is visible.  Everything a kernel does before pdl_wait() must touch no global
-// memory.  pdl_launch_dependents() lets the NEXT kernel on the stream start its own set-up as soon as
-// every CTA of this grid has executed it (or has exited).  Both are no-ops without the attribute.
+// memory, but for the decode kernel's reads of weights and weight scales that the caller declared static
+// (llmmm_set_static_weights).  pdl_launch_dependents() lets the NEXT kernel on the stream start its own set-up as
+// soon as every CTA of this grid has executed it (or has exited).  Both are no-ops without the attribute.
+//
+// A kernel executes it before its own pdl_wait(), so the kernel after the next one may start while this one is still
+// running, and only its pdl_wait() orders the two.  Kernels that write weights (the 128x128 quantiser, the transposes)
+// therefore do not execute it: nothing starts before they have completed, and an early read of a static weight finds
+// what they wrote, whatever small kernel lies between.  (They lose nothing: the next grid's waiting CTAs took SM slots
+// from theirs, 2048x1024 quantised 5.31 us with it and 4.60 without, a 19456x2560 weight prepared 121.8 and 121.0.)
 __device__ __forceinline__ void pdl_launch_dependents()
 {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

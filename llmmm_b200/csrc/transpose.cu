@@ -22,8 +22,7 @@ namespace llmmm {
 __global__ void __launch_bounds__(256) transpose_b32_kernel(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, int M, int N)
 {
   __shared__ uint4 T[64][16];
-  pdl_launch_dependents();  // see sm100.cuh: the next kernel may start its set-up, this one waits for its predecessor
-  pdl_wait();
+  pdl_wait();  // (no pdl_launch_dependents() in the kernels of this file: they write weights, see sm100.cuh)
   const int tx = threadIdx.x % 16;  // 4-column block of the input tile
   const int ry = threadIdx.x / 16;  // 4-row block
   const int m0 = blockIdx.y * 64;
@@ -50,7 +49,6 @@ __global__ void __launch_bounds__(256) transpose_b32_kernel(uint32_t* __restrict
 __global__ void __launch_bounds__(256) transpose_b32_small_kernel(uint32_t* __restrict__ dst, const uint32_t* __restrict__ src, int M, int N)
 {
   __shared__ uint32_t tile[32][33];
-  pdl_launch_dependents();
   pdl_wait();
   const int tx = threadIdx.x & 31;
   const int ty = threadIdx.x >> 5;
@@ -85,7 +83,6 @@ __device__ __forceinline__ uint4 transpose_4x4_bytes(uint32_t r0, uint32_t r1, u
 __global__ void __launch_bounds__(256) transpose_b8_kernel(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src, int M, int N)
 {
   __shared__ uint4 T[128 * 8];
-  pdl_launch_dependents();
   pdl_wait();
   const int tx = threadIdx.x & 7;   // 16-byte column block of the input tile
   const int ry = threadIdx.x >> 3;  // 4-row block

@@ -258,6 +258,45 @@ def test_decode_launch_chain_with_static_weights(capi, oracle, cuda, M):
         check_against_oracle(oracle, *case, promised[i][0].cpu().numpy(), promised[i][1].cpu().numpy(), Cf.cpu().numpy())
 
 
+@pytest.mark.parametrize("M", [1, 64])
+@pytest.mark.parametrize("NK", [(19456, 2560), (2560, 9728)])
+def test_static_weights_written_by_the_kernel_before_the_last(capi, cuda, M, NK):
+    # weight transposed or quantised, activations quantised, decode GEMM, with nothing in between: the early reads of the
+    # GEMM find the new weight and its scales
+    N, K = NK
+    g = torch.Generator(device=cuda).manual_seed(64)
+    x = torch.randn(M, K, device=cuda, generator=g)
+    w = [torch.randn(N, K, device=cuda, generator=g) * s for s in (0.02, 3.0)]
+    A_q, A_s = torch.empty(M, K, dtype=torch.uint8, device=cuda), torch.empty(K // 128, M, device=cuda)
+    B_q, B_s = torch.empty(N, K, dtype=torch.uint8, device=cuda), torch.empty(N // 128, K // 128, device=cuda)
+    B_t, B_kn = torch.empty_like(B_q), [torch.randint(0, 120, (K, N), dtype=torch.uint8, device=cuda, generator=g) for _ in range(2)]
+    C = torch.empty(M, N, device=cuda)
+    capi.ensure_workspace(M, N, K)
+
+    def call(i, wait):
+        outs = []
+        for quantised in (True, False):
+            if quantised:
+                capi.fp8_quant_128x128(w[i], B_q, B_s, N, K)
+            else:
+                capi.transpose_aligned_128(B_t, B_kn[i], K, N)
+            wait()
+            capi.fp8_quant_1x128(x, A_q, A_s, M, K)
+            capi.fp8_blockwise_mm_f32(A_q, A_s, B_q if quantised else B_t, B_s, C, M, N, K)
+            outs.append(C.clone())
+        return outs
+
+    expected = [call(i, torch.cuda.synchronize) for i in range(2)]
+    capi.set_static_weights(True)
+    try:
+        for rep in range(10):
+            for a, b in zip(call(rep & 1, lambda: None), expected[rep & 1]):
+                assert torch.equal(a, b)
+    finally:
+        capi.set_static_weights(False)
+    capi.check_status()
+
+
 @pytest.mark.parametrize("shape", [(128, 2560, 4096), (65, 512, 2048), (100, 4096, 1024)])
 def test_mid_m_few_tiles_take_the_pair_kernel_with_scratch(capi, oracle, cuda, shape):
     # 65..128 rows, tiles on at most half of the SMs: single-CTA kernel without scratch, pair kernel (whose tiles
