@@ -129,13 +129,29 @@ def test_swiglu_decode_sized(capi, oracle, cuda, M, IK):
     assert np.array_equal(gq2, gq3) and np.array_equal(gs2.view(np.uint32), gs3.view(np.uint32))
 
 
-@pytest.mark.parametrize("shape", [(65, 1152, 384), (128, 9728, 256), (100, 9472, 256), (300, 2560, 512)])
-def test_swiglu_128_row_tiles(capi, oracle, cuda, shape):
-    # the 128-row pair kernel's form: one and two waves of tiles, rows beyond the matrix in either CTA of a pair
+def kernel_of(call):
+    """Name of the one CUDA kernel that `call` launches."""
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
+        call()
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if "fp8_" in e.name]
+    assert len(names) == 1, names
+    return names[0]
+
+
+@pytest.mark.parametrize("shape,rows_per_tile", [((65, 1152, 384), 128), ((100, 9472, 256), 128), ((300, 2560, 512), 128), ((128, 9728, 256), 256),
+                                                 ((100, 9728, 2560), 128), ((128, 9728, 1792), 128)])
+def test_swiglu_128_row_tiles(capi, oracle, cuda, shape, rows_per_tile):
+    # the 128-row pair kernel's form: one wave of tiles and two (76 tiles on 74 pairs; with few K-blocks two such waves lose to
+    # the 256-row kernel), rows beyond the matrix in either CTA of a pair, K-blocks beyond the operand and the scale ring
     M, I, K = shape
     case = make_case(oracle, 96, M, I, K)
+    dev = to_dev(cuda, *case)
+    Hq, Hs = torch.empty((M, I), dtype=torch.uint8, device=cuda), torch.empty((I // 128, M), device=cuda)
+    name = kernel_of(lambda: capi.fp8_blockwise_mm_swiglu(*dev, Hq, Hs, M, I, K))
+    assert ("pair_kernel_m128" in name) == (rows_per_tile == 128), name
     gq, gs = run(capi, cuda, case, M, I, K)
-    check(oracle, case, gq, gs)
+    check(oracle, case, gq, gs, rows=None if I * K < 1 << 22 else (M - 3, 3))
     gq2, gs2 = run(capi, cuda, case, M, I, K)
     assert np.array_equal(gq, gq2) and np.array_equal(gs, gs2)
 
