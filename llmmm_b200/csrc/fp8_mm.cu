@@ -2074,7 +2074,6 @@ int launch_fp8_e4m3(const void* A, const float* A_s, const void* B, const float*
 
 int warm_fp8_kernels(const DeviceInfo* info)
 {
-  (void)info;
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_E4M3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_E4M3)));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_F32)));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel<EPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8pair::smem_bytes_of(EPI_SWIGLU)));
@@ -2087,6 +2086,9 @@ int warm_fp8_kernels(const DeviceInfo* info)
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_SWIGLU, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_GATHER, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_pair_kernel_m128<EPI_GATHER, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8p128::SMEM_BYTES));
+  for (int ways = 2; ways <= fp8p128::MAX_WAYS; ++ways) {
+    pair128_capacity(info, ways);  // occupancy queries, cached
+  }
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8cfg::SMEM_BYTES));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp8_blockwise_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp8cfg::SMEM_BYTES));
   return warm_decode_kernels(info);
