@@ -338,8 +338,8 @@ def main() -> int:
     achieved = FLOP_PER_STEP / (ms_step * 1e-3) / 1e12
     roofline = {
         "bound": "tensor", "achieved": achieved, "peak": fp8_peak, "unit": "TFLOP/s", "frac": achieved / fp8_peak,
-        "traffic": 37.7e6,
-        "traffic_source": "dram__bytes_read.sum 34.13 MB + dram__bytes_write.sum 3.55 MB of one launch of this kernel on this "
+        "traffic": 37.3e6,
+        "traffic_source": "dram__bytes_read.sum 34.13 MB + dram__bytes_write.sum 3.16 MB of one launch of this kernel on this "
                           "workload, from one ncu --set full capture (not re-measured by this run)",
         "peak_source": f"2 x bf16_tflops ({peak_kind}; the file has no fp8 figure; burst, kernel timed alone)",
         "frac_of_nominal_4500": achieved / 4500.0,

@@ -210,12 +210,14 @@ int llmmm_transpose_aligned_128(void* dst, const void* src, int M, int N, int el
 /* Split-K scratch.  The reference has no split-K (README.md:22 lists it as to
  * do) and its launchers allocate nothing, so the scratch is caller-owned: bytes
  * needed for a given problem, and registration of a device buffer for the
- * current device.  Two paths use it: the decode-sized (M <= 64) FP8 kernel, and,
- * for M > 128, the FP8 and FP16/BF16 kernels when their last wave of 256x256
- * tiles would leave most of the GPU idle: those tiles are then cut along K, the
- * fp32 partial tiles go through the scratch and are added in a fixed order
- * (results are bitwise stable from call to call, and differ from the unsplit
- * ones only by the association of fp32 sums).  llmmm_fp8_workspace_bytes gives
+ * current device.  Two paths use it: the decode-sized (M <= 64) FP8 kernel and
+ * hooks, and, for M > 128 (FP16/BF16: M > 64), the kernels with 256x256 tiles
+ * when their last wave would leave most of the GPU idle: those tiles are then
+ * cut along K, the fp32 partial tiles go through the scratch and are added in a
+ * fixed order (results are bitwise stable from call to call, and differ from the
+ * unsplit ones only by the association of fp32 sums).  With scratch registered,
+ * FP8 problems of M > 64 with few tiles run on 128x256 tiles instead, cut along K
+ * on chip; such a call leaves the scratch alone.  llmmm_fp8_workspace_bytes gives
  * the size for an FP8 problem; for FP16/BF16 pass the same M (any N, K >= 128).
  * Without registered scratch every shape still runs, unsplit.  llmmm_set_workspace
  * clears the parts of the buffer that must be zero between launches (it
@@ -344,8 +346,8 @@ int llmmm_tune(int kind, int N, int K);
 /* Number of kernels launched by this library in the calling process. */
 uint64_t llmmm_launch_count(void);
 
-/* How many of those launches cut the tiles of their last wave along K (possible for M > 128 once scratch
- * is registered with llmmm_set_workspace; see there).  A diagnostic: lets a caller see that its scratch
+/* How many of those launches cut tiles along K (possible for M > 64 once scratch is registered with
+ * llmmm_set_workspace; see there).  A diagnostic: lets a caller see that its scratch
  * registration took effect.  No counterpart in the reference. */
 uint64_t llmmm_split_launch_count(void);
 

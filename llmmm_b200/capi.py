@@ -1,4 +1,4 @@
-"""ctypes binding of the C ABI declared in include/llmmm_c.h.
+"""Python binding of the C ABI declared in include/llmmm_c.h.
 
 The functions here mirror the reference's host launchers (argument order and
 error behaviour): `fp16_mm` is LLMMM::fp16_mm<T> (src/mm/fp16/mm.h:9-10), the
@@ -126,7 +126,7 @@ def launch_count() -> int:
 
 
 def split_launch_count() -> int:
-    """Launches so far that cut the tiles of their last wave along K (needs registered scratch)."""
+    """Launches so far that cut tiles along K (needs registered scratch)."""
     return int(lib().llmmm_split_launch_count())
 
 

@@ -469,11 +469,13 @@ struct Fp8PairBars {
 //   EPI_ROPE   like EPI_E4M3 for a qkv projection with heads of 128 columns: a thread's 128 accumulators are one
 //              head of its row, so the per-head RMSNorm of query / key heads and the rotary embedding are
 //              thread-local arithmetic in front of the quantisation.
-// Which general kernel a problem runs on.  More than 128 rows: the pair kernel.  65..128 rows: the single-CTA
-// kernel (128-row tiles waste nothing), unless its tiles would occupy at most half of the SMs and scratch is
-// registered: then the pair kernel, whose tiles can be cut along K, wins although half of each tile's rows are
-// empty (measured at M = 128: 2560x9728 45.6 -> 23.6 us, 4096x4096 21.5 -> 18.2 us; 19456x2560, 76 tiles,
-// would lose: 17.3 -> 29.3 us).
+// Which general kernel a problem runs on.  More than 128 rows: a pair kernel.  65..128 rows: the single-CTA kernel
+// while its 128x256 tiles occupy more than half of the SMs, else a pair of SMs per tile (the 128-row pair kernel, with
+// fewer tiles several pairs) is faster: M = 128, 2560x9728 45.6 -> 13.5 us, 4096x4096 21.7 -> 11.4, 6144x2560 15.3 ->
+// 10.3, 9216x1280 10.0 -> 7.0, 9472x2560 (37 tiles) 15.5 -> 9.8; 19456x2560, 76 tiles on 74 pairs, takes 16.8 us on
+// the single-CTA kernel, which llmmm_tune finds the faster of the two.  The pair kernels are chosen only with scratch
+// registered, as when the 256-row one (which needs it to cut tiles) was the alternative: without scratch a call of so
+// few rows sums as it always did.
 // With K given, a choice llmmm_tune measured for this weight shape takes precedence (as long as the scratch the
 // pair kernel's split needs is there).
 static bool fp8_use_pair_kernel(const DeviceInfo* info, int M, int N, int K = 0, bool* tuned = nullptr)
@@ -1822,8 +1824,8 @@ static bool pair128_folds(const DeviceInfo* info, int M, int N, int K, int ways)
 // Whether a problem that is the pair kernels' runs with 128-row tiles.  Up to 128 rows always.  Above, a 128-row tile has
 // half the work at about 0.6 of the time per K-block (0.3-0.36 against 0.55 us), so it wins where its tiles (cut along K or
 // not) fit on the pairs at once and those of 256 rows leave pairs idle or are cut; the fixed costs are 3.8 and 5 us, cutting
-// costs 2.5 us here and about 3 + 1.5 per way there.  Measured, 256-row against 128-row tiles: 256x2560x9728 23.5 / 15.5 us,
-// 256x6144x2560 15.4 / 9.9, 512x4096x4096 18.9 / 13.5, 700x2560x4096 18.7 / 13.4.  Beyond 768 rows only tiles that are
+// costs 2.5 us here and about 3 + 1.5 per way there.  Measured, 256-row against 128-row tiles: 256x2560x9728 23.5 / 16.3 us,
+// 256x6144x2560 15.3 / 9.9, 512x4096x4096 19.0 / 14.1, 700x2560x4096 18.6 / 14.0.  Beyond 768 rows only tiles that are
 // cut: callers are told (llmmm_split_launch_count, llmmm_c.h) that the last wave of such a problem is cut along K when
 // scratch is registered.
 static bool use_pair128(const DeviceInfo* info, int M, int N, int K)
