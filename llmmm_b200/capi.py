@@ -18,21 +18,27 @@ torch in use.
 from __future__ import annotations
 
 import ctypes
+import importlib
 import sys
 import warnings
 from pathlib import Path
 
 import torch
 
-try:
-    from . import _binding as _native
-    _built_for = getattr(_native, "BUILT_FOR", "another torch")
-    _native_missing = "" if _built_for == f"torch {torch.__version__}, python {sys.version_info.major}.{sys.version_info.minor}" \
-        else f"it was built for {_built_for}"
-except ImportError as e:
-    _native_missing = str(e)
-if _native_missing:
-    _native = None
+
+def _load_native():
+    """(_binding, "") or (None, why not)."""
+    try:
+        binding = importlib.import_module("._binding", __package__)
+    except ImportError as e:
+        return None, str(e)
+    built_for = getattr(binding, "BUILT_FOR", "another torch")
+    if built_for != f"torch {torch.__version__}, python {sys.version_info.major}.{sys.version_info.minor}":
+        return None, f"it was built for {built_for}"
+    return binding, ""
+
+
+_native, _native_missing = _load_native()
 
 _LIB_PATH = Path(__file__).resolve().parent / "libllmmm_b200.so"
 _lib = None
@@ -43,11 +49,13 @@ _i = ctypes.c_int
 
 def lib() -> ctypes.CDLL:
     """Loads libllmmm_b200.so (built in-tree by llmmm_b200.build)."""
-    global _lib
+    global _lib, _native, _native_missing
     if _lib is None:
         if not _LIB_PATH.exists():
             raise RuntimeError(
                 f"{_LIB_PATH} is missing: build it with `python -m llmmm_b200.build`; there is no fallback path")
+        if _native is None:  # (the package may have been imported before it was built)
+            _native, _native_missing = _load_native()
         if _native is None:
             warnings.warn(f"_binding.so is not used ({_native_missing}): calls cost the host about three times as much; build it with "
                           "`python -m llmmm_b200.build`", stacklevel=2)
