@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(fp16cfg::THREADS, 1) fp16_gemm_kernel(const __
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer --
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
         const int m0 = (tile % m_tiles) * BM;
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(fp16cfg::THREADS, 1) fp16_gemm_kernel(const __
   }
   else if (warp == 1) {
     // -------------------------------------------------------- MMA issuer --
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t kFmt  = std::is_same<T, __half>::value ? 0u : 1u;
       constexpr uint32_t idesc = make_idesc(kFmt, kFmt, /*a_mn=*/0, /*b_mn=*/1, BM, BN);
       uint32_t           it    = 0;
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(fp16pair::THREADS, 1)
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer --
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       PairWalk walk(pair, n_pairs, k_iters, dp_tiles, split_pairs, split_s, split_chunk);
       int      tile, kb0, kb1;
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(fp16pair::THREADS, 1)
   }
   else if (warp == 1) {
     // ------------------------------------------- MMA issuer (leader only) --
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t kFmt  = std::is_same<T, __half>::value ? 0u : 1u;
       constexpr uint32_t idesc = make_idesc(kFmt, kFmt, /*a_mn=*/0, /*b_mn=*/1, BM, BN);
       uint32_t           it    = 0;

@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
     // of the stream: the first ring of weight tiles is requested before waiting for that kernel, the
     // activation tiles of the same stages after it.
     uint32_t early = 0;
-    if (lane == 0 && early_weights) {
+    if (early_weights && elect_one()) {
       walk([&](uint32_t it, int nb, int kb) {
         if (it >= (uint32_t)L::STAGES) {
           return false;
@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
     }
     __syncwarp();
     pdl_wait();
-    if (lane == 0) {
+    if (elect_one()) {
       walk([&](uint32_t it, int nb, int kb) {
         const uint32_t s  = it % L::STAGES;
         const uint32_t ph = (it / L::STAGES) & 1;
@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
     // --------------------------------------------- three MMA issuers ------
     // Warps 1, 2 and 3 take every third K-block of the run; each K-block has its own ring slot and
     // tensor-memory partial stage, so the threads never touch the same barrier phase.
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, 128, MP);
       for (uint32_t it = (uint32_t)(warp - 1); it < run; it += 3) {
         const uint32_t s  = it % L::STAGES;

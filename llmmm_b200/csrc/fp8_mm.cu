@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(fp8cfg::THREADS, 1) fp8_blockwise_gemm_kernel(
     setmaxnreg_dec<REGS_CTRL>();
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer --
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
         const int m0 = (tile % m_tiles) * BM;
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(fp8cfg::THREADS, 1) fp8_blockwise_gemm_kernel(
   }
   else if (warp == 1) {
     // -------------------------------------------------------- MMA issuer --
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, BM, BN);
       uint32_t           it    = 0;
       for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
     setmaxnreg_dec<REGS_CTRL>();
     if (warp == 0) {
       // ---------------------------------------------------- TMA producer --
-      if (lane == 0) {
+      if (elect_one()) {
         uint32_t it = 0;
         PairWalk walk(pair, n_pairs, k_blocks, dp_tiles, split_pairs, split_s, split_chunk);
         int      tile, kb0, kb1;
@@ -720,7 +720,7 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
       // threads issuing alternate groups reach the full 129 clk), and it cannot poll the barriers of
       // the next K-block meanwhile.  Two threads take alternate K-blocks (each owns one TMEM partial
       // stage): one sits in its barrier waits while the MMAs of the other run.
-      if (lane == 0 && rank == 0) {
+      if (rank == 0 && elect_one()) {
         constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, BM, BN);
         const uint32_t     p     = (warp == 1) ? 0u : 1u;  // partial stage and K-block parity of this thread
 #ifdef LLMMM_PROFILE
@@ -1395,7 +1395,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
     setmaxnreg_dec<regs_ctrl(FOLDS)>();
     if (warp == 0) {
       // ---------------------------------------------------- TMA producer --
-      if (lane == 0) {
+      if (elect_one()) {
         uint32_t s = 0, ph = 0;
         for (int kb = kb0; kb < kb1; ++kb) {
           mbar_wait(&bars->done[s], ph ^ 1, DEV_WAIT_SMEM_EMPTY, abort_flag, status);
@@ -1433,7 +1433,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
       }
       cp_async_wait_all();
     }
-    else if (lane == 0 && rank == 0) {
+    else if (rank == 0 && elect_one()) {
       // ------------------------------------ two MMA issuers (leader only) --
       constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, BM, BN);
       const uint32_t     total = (uint32_t)(kb1 - kb0);
