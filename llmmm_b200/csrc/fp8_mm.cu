@@ -77,12 +77,42 @@ struct Fp8Bars {
   uint32_t abort_flag;
 };
 
-// acc{0,1} = fma(v{0,1}, sc, acc{0,1}).  Two scalar FMAs: the packed fma.rn.f32x2 has the same flop rate
-// and was measured slower here (aligned register pairs cost registers in a loop that has none to spare).
+// acc{0,1} = fma(v{0,1}, sc, acc{0,1}) as one packed instruction, the same two roundings.  A warp's stream of scalar FMAs
+// takes every issue slot of its scheduler and the control warp beside it gets almost none (MMAs issued beside two such
+// warps per scheduler: 2500 clk per K-block of 514 clk of tensor work); the packed form leaves slots free and the
+// control warps run at full speed (514 clk).
+__device__ __forceinline__ void ffma2(float& d0, float& d1, uint32_t a0, uint32_t a1, uint64_t sc)
+{
+  asm("{\n\t"
+      ".reg .b64 d, a;\n\t"
+      "mov.b64 d, {%0, %1};\n\t"
+      "mov.b64 a, {%2, %3};\n\t"
+      "fma.rn.f32x2 d, a, %4, d;\n\t"
+      "mov.b64 {%0, %1}, d;\n\t"
+      "}"
+      : "+f"(d0), "+f"(d1)
+      : "r"(a0), "r"(a1), "l"(sc));
+}
+
+// The same as two scalar instructions, where register pairs spill (a few bytes spilt in a promotion loop cost more).
 __device__ __forceinline__ void ffma2(float& d0, float& d1, uint32_t a0, uint32_t a1, float sc)
 {
   d0 = __fmaf_rn(__uint_as_float(a0), sc, d0);
   d1 = __fmaf_rn(__uint_as_float(a1), sc, d1);
+}
+
+// The scale as ffma2() takes it: twice in a register pair (packed) or as it is.
+template<bool PACKED>
+__device__ __forceinline__ auto scale_operand(float sc)
+{
+  if constexpr (PACKED) {
+    uint64_t p;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(p) : "f"(sc));
+    return p;
+  }
+  else {
+    return sc;
+  }
 }
 
 // largest magnitude of a thread's 128 accumulators, in four chains (one chain is 128 dependent instructions)
@@ -267,8 +297,7 @@ __global__ void __launch_bounds__(fp8cfg::THREADS, 1) fp8_blockwise_gemm_kernel(
         float a_cur = a_pf[j], b_cur = b_pf[j];
         asm volatile("" : "+f"(a_cur), "+f"(b_cur));
         // one fp32 rounding of the scale product, as in the reference
-        const float    sc  = __fmul_rn(a_cur, b_cur);
-        const float    sc2 = sc;
+        const float scp = __fmul_rn(a_cur, b_cur);
         if (kb + PREFETCH < k_blocks) {
           a_pf[j] = __ldg(a_s + (size_t)(kb + PREFETCH) * M);
           b_pf[j] = __ldg(b_s + kb + PREFETCH);
@@ -282,19 +311,19 @@ __global__ void __launch_bounds__(fp8cfg::THREADS, 1) fp8_blockwise_gemm_kernel(
         tmem_ld_32x32b_x32(t_addr + 32, v1);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          ffma2(acc[i], acc[i + 1], v0[i], v0[i + 1], sc2);
+          ffma2(acc[i], acc[i + 1], v0[i], v0[i + 1], scp);
         }
         tmem_ld_wait();
         tmem_ld_32x32b_x32(t_addr + 64, v0);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          ffma2(acc[32 + i], acc[32 + i + 1], v1[i], v1[i + 1], sc2);
+          ffma2(acc[32 + i], acc[32 + i + 1], v1[i], v1[i + 1], scp);
         }
         tmem_ld_wait();
         tmem_ld_32x32b_x32(t_addr + 96, v1);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          ffma2(acc[64 + i], acc[64 + i + 1], v0[i], v0[i + 1], sc2);
+          ffma2(acc[64 + i], acc[64 + i + 1], v0[i], v0[i + 1], scp);
         }
         tmem_ld_wait();
         // every column of this thread's part of the partial stage has been read
@@ -305,7 +334,7 @@ __global__ void __launch_bounds__(fp8cfg::THREADS, 1) fp8_blockwise_gemm_kernel(
         }
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          ffma2(acc[96 + i], acc[96 + i + 1], v1[i], v1[i + 1], sc2);
+          ffma2(acc[96 + i], acc[96 + i + 1], v1[i], v1[i + 1], scp);
         }
         ++it;
       }
@@ -372,14 +401,22 @@ __global__ void __launch_bounds__(fp8cfg::THREADS, 1) fp8_blockwise_gemm_kernel(
 //
 // The same computation for a cluster of two CTAs that share one 256x256 output
 // tile (tcgen05.mma.cta_group::2), used when M > 128.  CTA r loads its own 128
-// rows of A_q and the 128 B_q rows of the tile's scale group r, so a CTA
-// streams 32 KB per K-block instead of 48 KB (6-stage ring) and its shared
-// memory serves 32 KB of operand reads per K-block instead of 48 KB.  Shared
-// memory bandwidth (TMA writes + MMA reads, about 128 B/clk) is what bounds the
-// single-CTA kernel.  Only the even CTA issues MMAs (256x256x32); both CTAs'
-// loads signal its `full` barrier, its commits arrive on both CTAs' `empty` and
-// `part_full` barriers, and both CTAs' promotion warps release a partial stage
-// by arriving on its `part_empty` barrier.
+// rows of A_q and 64 B_q rows of either scale group of the tile, so a CTA
+// streams 32 KB per K-block instead of 48 KB and its shared memory serves less
+// than the 128 B/clk (TMA writes + MMA reads) that bound the single-CTA kernel.
+// Only the even CTA issues MMAs; both CTAs' loads signal its `full` barrier, its
+// commits arrive on both CTAs' `done` barriers, and both CTAs' promotion warps
+// release a partial by arriving on its `part_empty` barrier.
+//
+// A K-block is issued as its two column halves (256x128x32 MMAs), each with
+// barriers of its own: two partial stages times two halves of 128 tensor-memory
+// columns.  With one group of 256 columns the four warps of a scheduler pair
+// found their partial at the same moment, loaded together and multiplied
+// together, and a stage came free only when the slowest of 16 warps had read it;
+// the halves are 257 clk apart.  Measured with packed FMAs and one issuing
+// thread in both: 4096^3 75.0 -> 73.6 us, Qwen3-4B layer of 1333 rows 210.7 ->
+// 204.9, 8192-row MLP 1669 -> 1624 (where the 1000 W cap decides: the same MMAs
+// with no promotion arithmetic at all take 0.86 of the time, at a lower clock).
 #ifdef LLMMM_PROFILE
 // Debug build only: cycle counters of CTA 0 (MMA thread: total, waiting for operands, waiting for a
 // free partial stage; promotion warp 4: waiting for a partial, epilogue), see llmmm_profile_dump8().
@@ -408,12 +445,13 @@ constexpr int      REGS_CTRL  = 40;  // (32 spilt in the promotion loop)
 constexpr int      REGS_PROMO = 232;
 static_assert(128 * REGS_CTRL + 256 * REGS_PROMO <= THREADS * 168, "setmaxnreg split exceeds the CTA's registers");
 constexpr uint32_t A_BYTES    = 128 * BK;                 // 16 KB: this CTA's rows
-constexpr uint32_t B_BYTES    = 128 * BK;                 // 16 KB: this CTA's half of the tile's columns
+constexpr uint32_t B_BYTES    = 128 * BK;                 // 16 KB: this CTA's 64 columns of either half of the tile
 constexpr uint32_t STAGE_TX   = 2 * (A_BYTES + B_BYTES);  // both CTAs' loads land on the leader's barrier
 // Ring of scale operands, filled by a warp of its own: a slot holds SC_KB K-blocks of this CTA's 128 A scales
-// followed by the tile's two B scales (SWIGLU: the gate rows' and the up rows').
-constexpr int      SC_KB      = 4;
-constexpr int      SC_SLOTS   = 4;
+// followed by the tile's two B scales (SWIGLU: the gate rows' and the up rows').  (Two slots of eight and not four of four:
+// going from slot to slot costs a promotion warp about 150 clk, 700 -> 670 clk per K-block at 8192x4096x8192.)
+constexpr int      SC_KB      = 8;
+constexpr int      SC_SLOTS   = 2;
 constexpr int      SC_ROW     = 132;  // floats per K-block: 128 + 2, padded to 16 bytes
 constexpr uint32_t SC_BYTES   = SC_SLOTS * SC_KB * SC_ROW * 4;
 // Shared memory, per epilogue (the EPI_* constants: 2 swiglu, 4 rope): operand ring | barriers | scale ring |
@@ -437,7 +475,7 @@ __host__ __device__ constexpr uint32_t off_sc(int epi) { return off_xch(epi) + x
 __host__ __device__ constexpr uint32_t off_bar(int epi) { return off_sc(epi) + SC_BYTES; }
 __host__ __device__ constexpr uint32_t smem_bytes_of(int epi) { return off_bar(epi) + 512 + 1024; }
 static_assert(smem_bytes_of(0) <= 232448 && smem_bytes_of(2) <= 232448 && smem_bytes_of(4) <= 232448, "shared memory of an SM");
-constexpr uint32_t TMEM_COLS  = 512;  // two partial stages of 256 columns
+constexpr uint32_t TMEM_COLS  = 512;  // two partial stages of two halves of 128 columns
 // split tiles (pair_walk.cuh): a slot holds 16 warp-sized units of 32 rows x 128 columns
 constexpr size_t   SK_UNIT_FLOATS = 32 * 128;
 static_assert(16 * SK_UNIT_FLOATS == SPLIT_SLOT_FLOATS, "one slot per 256x256 tile");
@@ -445,9 +483,9 @@ static_assert(16 * SK_UNIT_FLOATS == SPLIT_SLOT_FLOATS, "one slot per 256x256 ti
 
 struct Fp8PairBars {
   uint64_t full[6];        // used in the leader CTA
-  uint64_t done[6];        // both CTAs (multicast commit): the K-block's MMAs are done, so the ring slot is free and
-                           // the partial stage can be read (one commit per K-block serves both)
-  uint64_t part_empty[2];  // used in the leader CTA, 16 arrivals
+  uint64_t done[6][2];     // both CTAs (multicast commit): the MMAs of one column half of the K-block are done, so that half
+                           // of the partial stage can be read; the second half's also say that the ring slot is free
+  uint64_t part_empty[4];  // used in the leader CTA, 8 arrivals: partial stage p, column half h at 2 p + h
   uint64_t sc_full[fp8pair::SC_SLOTS];   // 32 arrivals: the scale warp's lanes, when their copies have landed
   uint64_t sc_empty[fp8pair::SC_SLOTS];  // 8 arrivals: the promotion warps
   uint32_t tmem_base;
@@ -616,10 +654,11 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < NSTAGES; ++s) {
       mbar_init(&bars->full[s], 1);
-      mbar_init(&bars->done[s], 1);
+      mbar_init(&bars->done[s][0], 1);
+      mbar_init(&bars->done[s][1], 1);
     }
-    for (int p = 0; p < 2; ++p) {
-      mbar_init(&bars->part_empty[p], 16);  // 8 promotion warps of each CTA
+    for (int p = 0; p < 4; ++p) {
+      mbar_init(&bars->part_empty[p], 8);  // the half's 4 promotion warps of each CTA
     }
     for (int i = 0; i < SC_SLOTS; ++i) {
       mbar_init(&bars->sc_full[i], 32);
@@ -655,36 +694,30 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
         int      tile, kb0, kb1;
         while (walk.next(tile, kb0, kb1)) {
           const int m0 = (tile % m_tiles) * BM + (int)rank * 128;
-          const int n0 = (tile / m_tiles) * TILE_N + (int)rank * (SWIGLU ? 64 : 128);
+          // B rows of column half h: of an MMA's 128 columns the leader supplies 64 and its partner 64 (SWIGLU: the gate rows
+          // and the up rows of the same output columns)
+          const int n0 = (tile / m_tiles) * TILE_N + (int)rank * (SWIGLU ? N : 64);
           for (int kb = kb0; kb < kb1; ++kb, ++it) {
             const uint32_t s  = it % NSTAGES;
             const uint32_t ph = (it / NSTAGES) & 1;
-            mbar_wait(&bars->done[s], ph ^ 1, DEV_WAIT_SMEM_EMPTY, abort_flag, status);
+            mbar_wait(&bars->done[s][1], ph ^ 1, DEV_WAIT_SMEM_EMPTY, abort_flag, status);
             const uint32_t full_leader = mapa_shared(smem_u32(&bars->full[s]), 0);
             if (rank == 0) {
               mbar_arrive_expect_tx(&bars->full[s], STAGE_TX);
             }
             tma_load_2d_pair(smem + OFF_A + s * A_BYTES, &tm_a, full_leader, kb * BK, m0);
-            if constexpr (SWIGLU) {
-              // 64 gate rows, then the 64 up rows of the same output columns (the B descriptor's box is 64 rows)
-              tma_load_2d_pair(smem + OFF_B + s * B_BYTES, &tm_b, full_leader, kb * BK, n0);
-              tma_load_2d_pair(smem + OFF_B + s * B_BYTES + B_BYTES / 2, &tm_b, full_leader, kb * BK, N + n0);
-            }
-            else {
-              tma_load_2d_pair(smem + OFF_B + s * B_BYTES, &tm_b, full_leader, kb * BK, n0);
-            }
+            tma_load_2d_pair(smem + OFF_B + s * B_BYTES, &tm_b, full_leader, kb * BK, n0);
+            tma_load_2d_pair(smem + OFF_B + s * B_BYTES + B_BYTES / 2, &tm_b, full_leader, kb * BK, n0 + (SWIGLU ? 64 : 128));
           }
         }
       }
     }
     else if (warp == 2) {
       // ---------------------------------------------------- scale operands --
-      // The promotion warps must never wait for global memory: the slowest of the 16 warps of a pair decides when a
-      // partial stage can be written again, and under the operand traffic an L2 hit takes one to two K-blocks.  This
+      // The promotion warps must never wait for global memory: the slowest of the 8 warps of a half decides when its
+      // partial can be written again, and under the operand traffic an L2 hit takes one to two K-blocks.  This
       // warp therefore copies the scales up to SC_SLOTS * SC_KB K-blocks ahead.  (Copies of 4 bytes: a row of A_s
-      // starts at a multiple of 16 bytes only if M is a multiple of 4.)  While every promotion thread fetched its own
-      // scales two K-blocks ahead, a K-block took 1078 clk at 4096^3 and 1458 clk at 8192x4096x8192; with the ring
-      // (and one commit per K-block instead of two) 943 and 911.
+      // starts at a multiple of 16 bytes only if M is a multiple of 4.)
       uint32_t c = 0;
       PairWalk walk(pair, n_pairs, k_blocks, dp_tiles, split_pairs, split_s, split_chunk);
       int      tile, kb0, kb1;
@@ -713,62 +746,61 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
       }
       cp_async_wait_all();
     }
-    else {
-      // ------------------------------------ two MMA issuers (leader only) --
-      // A thread that issues a group of MMAs followed by tcgen05.commit is held for about the
-      // duration of the group (measured: one thread feeds the pipe at 160-190 clk per MMA, two
-      // threads issuing alternate groups reach the full 129 clk), and it cannot poll the barriers of
-      // the next K-block meanwhile.  Two threads take alternate K-blocks (each owns one TMEM partial
-      // stage): one sits in its barrier waits while the MMAs of the other run.
+    else if (warp == 1) {
+      // ------------------------------------------- MMA issuer (leader only) --
       if (rank == 0 && elect_one()) {
-        constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, BM, BN);
-        const uint32_t     p     = (warp == 1) ? 0u : 1u;  // partial stage and K-block parity of this thread
+        constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, BM, 128);
 #ifdef LLMMM_PROFILE
         long long p_full = 0, p_part = 0, p_t0 = clock64();
         unsigned long long p_g0 = global_timer_ns();
 #endif
-        // the MMA threads need no tile identities, only the number of K-blocks this pair works through
+        // the MMA thread needs no tile identities, only the number of K-blocks this pair works through
         const uint32_t total = PairWalk(pair, n_pairs, k_blocks, dp_tiles, split_pairs, split_s, split_chunk).total_k_blocks();
-        for (uint32_t it = p; it < total; it += 2) {
-          {
-            const uint32_t s  = it % NSTAGES;
-            const uint32_t ph = (it / NSTAGES) & 1;
-            const uint32_t pp = (it >> 1) & 1;
-            PROF8_T(c0);
-            mbar_wait(&bars->part_empty[p], pp ^ 1, DEV_WAIT_TMEM_EMPTY, abort_flag, status);
-            PROF8_T(c1);
-            mbar_wait(&bars->full[s], ph, DEV_WAIT_SMEM_FULL, abort_flag, status);
+        uint32_t       s = 0, ph = 0;
+        for (uint32_t it = 0; it < total; ++it) {
+          const uint32_t p = it & 1;
+          PROF8_T(c0);
+          mbar_wait(&bars->full[s], ph, DEV_WAIT_SMEM_FULL, abort_flag, status);
+          PROF8_T(c1);
+          PROF8_ADD(p_full, c0, c1);
+#ifdef LLMMM_PROFILE
+          if (blockIdx.x == 0 && it < 64) {
+            g_trace8[it][0] = c0;  // MMA thread: starts waiting for the operands
+            g_trace8[it][1] = c1;  // operands present
+          }
+#endif
+          const uint64_t da = make_smem_desc_sw128(smem_u32(smem + OFF_A + s * A_BYTES), 0, 1024);
+          const uint64_t db = make_smem_desc_sw128(smem_u32(smem + OFF_B + s * B_BYTES), 0, 1024);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            PROF8_T(c3);
+            mbar_wait(&bars->part_empty[2 * p + h], ((it >> 1) & 1) ^ 1, DEV_WAIT_TMEM_EMPTY, abort_flag, status);
             PROF8_T(c2);
-            PROF8_ADD(p_part, c0, c1);
-            PROF8_ADD(p_full, c1, c2);
+            PROF8_ADD(p_part, c3, c2);
 #ifdef LLMMM_PROFILE
             if (blockIdx.x == 0 && it < 64) {
-              g_trace8[it][0] = c0;  // MMA thread: starts waiting for the partial stage
-              g_trace8[it][1] = c1;  // partial stage free
-              g_trace8[it][2] = c2;  // operands present
+              g_trace8[it][2 + h] = c2;  // half of the partial stage free
             }
 #endif
             tc_fence_after_sync();
-            const uint64_t da = make_smem_desc_sw128(smem_u32(smem + OFF_A + s * A_BYTES), 0, 1024);
-            const uint64_t db = make_smem_desc_sw128(smem_u32(smem + OFF_B + s * B_BYTES), 0, 1024);
 #pragma unroll
             for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-              tc_mma_f8_pair(tmem_base + p * BN, da + (uint64_t)((kk * UMMA_K) >> 4), db + (uint64_t)((kk * UMMA_K) >> 4), idesc, kk != 0);
+              tc_mma_f8_pair(tmem_base + p * BN + h * 128, da + (uint64_t)((kk * UMMA_K) >> 4),
+                             db + (uint64_t)((h * (B_BYTES / 2) + kk * UMMA_K) >> 4), idesc, kk != 0);
             }
-            tc_commit_pair(&bars->done[s]);
-#ifdef LLMMM_PROFILE
-            if (blockIdx.x == 0 && it < 64) {
-              g_trace8[it][3] = clock64();  // MMAs and commits issued
-            }
-#endif
+            tc_commit_pair(&bars->done[s][h]);
+          }
+          if (++s == NSTAGES) {
+            s = 0;
+            ph ^= 1;
           }
         }
 #ifdef LLMMM_PROFILE
-        if (blockIdx.x == 0 && p == 0) {
+        if (blockIdx.x == 0) {
           g_prof8[0] = clock64() - p_t0;
           g_prof8[1] = (long long)(global_timer_ns() - p_g0);
-          g_prof8[2] = 2 * p_full;
-          g_prof8[3] = 2 * p_part;
+          g_prof8[2] = p_full;
+          g_prof8[3] = p_part;
           g_prof8[4] = total;
         }
 #endif
@@ -787,9 +819,9 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
     // (barriers are addressed by 32-bit shared-memory addresses: the loop has no register to spare)
     const uint32_t bars_at      = smem_u32(bars);
     const uint32_t abort_at     = smem_u32(&bars->abort_flag);
-    const uint32_t empty_leader = mapa_shared(smem_u32(&bars->part_empty[0]), 0);
+    const uint32_t empty_leader = mapa_shared(smem_u32(&bars->part_empty[half]), 0);
     uint32_t       it           = 0;
-    uint32_t       done_at = bars_at + (uint32_t)offsetof(Fp8PairBars, done), done_ph = 0;  // of K-block `it`
+    uint32_t       done_at = bars_at + (uint32_t)offsetof(Fp8PairBars, done) + half * 8, done_ph = 0;  // of K-block `it`
     uint32_t       sc_slot = 0, sc_ph = 0;
     const uint32_t sc_mine = smem_u32(sc_ring) + (quarter * 32 + lane) * 4;  // this thread's row in slot 0 ...
     const uint32_t sc_b    = (128 - quarter * 32 - lane + (SWIGLU ? 0 : half)) * 4;  // ... and from there to its B scale
@@ -860,8 +892,7 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
           const uint32_t p = it & 1;
           // one fp32 rounding of the scale product, as in the reference
           const float a_cur    = lds_f32(sc_addr);
-          const float sc2      = __fmul_rn(a_cur, lds_f32(sc_addr + sc_b));
-          float       sc2_late = SWIGLU ? __fmul_rn(a_cur, lds_f32(sc_addr + sc_b + 4)) : sc2;  // of the last 64 accumulators (SWIGLU: the up rows')
+          const uint64_t scp = scale_operand<true>(__fmul_rn(a_cur, lds_f32(sc_addr + sc_b)));
           PROF8_T(d0);
           mbar_wait_at(done_at, done_ph, DEV_WAIT_TMEM_FULL, abort_at, status);
           PROF8_T(d1);
@@ -881,20 +912,24 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            ffma2(acc[i], acc[i + 1], v0[i], v0[i + 1], sc2);
+            ffma2(acc[i], acc[i + 1], v0[i], v0[i + 1], scp);
           }
           tmem_ld_32x32b_x32(t_addr + 64, v0);
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            ffma2(acc[32 + i], acc[32 + i + 1], v1[i], v1[i + 1], sc2);
+            ffma2(acc[32 + i], acc[32 + i + 1], v1[i], v1[i + 1], scp);
           }
           tmem_ld_32x32b_x32(t_addr + 96, v1);
+          uint64_t scl = scp;  // of the last 64 accumulators
+          if constexpr (SWIGLU) {
+            scl = scale_operand<true>(__fmul_rn(a_cur, lds_f32(sc_addr + sc_b + 4)));  // ... the up rows'
+          }
           tmem_ld_wait();
           // every column of this thread's part of the partial stage has been read
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) {
-            mbar_arrive_cluster_relaxed(empty_leader + p * 8);
+            mbar_arrive_cluster_relaxed(empty_leader + p * 16);
           }
 #ifdef LLMMM_PROFILE
           if (blockIdx.x == 0 && threadIdx.x == 128 && it < 64) {
@@ -904,19 +939,24 @@ __global__ void __launch_bounds__(fp8pair::THREADS, 1)
           // The arithmetic on the last two loads must stay behind the hand-back above: the compiler may
           // move plain FMAs across asm statements, but not asm volatile statements across one another, so
           // the scale is passed through an empty one.
-          asm volatile("" : "+f"(sc2_late));
+          asm volatile("" : "+l"(scl));
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            ffma2(acc[64 + i], acc[64 + i + 1], v0[i], v0[i + 1], sc2_late);
+            ffma2(acc[64 + i], acc[64 + i + 1], v0[i], v0[i + 1], scl);
           }
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            ffma2(acc[96 + i], acc[96 + i + 1], v1[i], v1[i + 1], sc2_late);
+            if constexpr (SWIGLU || EPI == EPI_ROPE) {
+              ffma2(acc[96 + i], acc[96 + i + 1], v1[i], v1[i + 1], __uint_as_float((uint32_t)scl));  // (pairs throughout spill here)
+            }
+            else {
+              ffma2(acc[96 + i], acc[96 + i + 1], v1[i], v1[i + 1], scl);
+            }
           }
           ++it;
-          done_at += 8;
-          if (done_at == bars_at + (uint32_t)offsetof(Fp8PairBars, done) + NSTAGES * 8) {
-            done_at -= NSTAGES * 8;
+          done_at += 16;
+          if (done_at >= bars_at + (uint32_t)offsetof(Fp8PairBars, done) + NSTAGES * 16) {
+            done_at -= NSTAGES * 16;
             done_ph ^= 1;
           }
         }
@@ -1272,11 +1312,9 @@ constexpr int      BK         = 128;
 constexpr int      UMMA_K     = 32;
 constexpr uint32_t STAGES     = 7;
 constexpr int      THREADS    = 384;
-// (a form with folds, see below, spilt in the control warps with 64)
-__host__ __device__ constexpr int regs_ctrl(bool folds) { return folds ? 72 : 56; }
-__host__ __device__ constexpr int regs_promo(bool folds) { return folds ? 216 : 224; }
-static_assert(128 * regs_ctrl(true) + 256 * regs_promo(true) <= THREADS * 168, "setmaxnreg split exceeds the CTA's registers");
-static_assert(128 * regs_ctrl(false) + 256 * regs_promo(false) <= THREADS * 168, "setmaxnreg split exceeds the CTA's registers");
+constexpr int      REGS_CTRL  = 72;   // (with 64 the form with folds, see below, spilt in the control warps)
+constexpr int      REGS_PROMO = 216;
+static_assert(128 * REGS_CTRL + 256 * REGS_PROMO <= THREADS * 168, "setmaxnreg split exceeds the CTA's registers");
 constexpr uint32_t A_BYTES    = 64 * BK;
 constexpr uint32_t B_BYTES    = 128 * BK;
 constexpr uint32_t STAGE_TX   = 2 * (A_BYTES + B_BYTES);
@@ -1335,6 +1373,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
   using namespace fp8p128;
   constexpr bool OUT_F32 = EPI == EPI_F32, SWIGLU = EPI == EPI_SWIGLU;
   constexpr bool BY_ROW  = EPI != EPI_F32 && EPI != EPI_E4M3;  // rows are finished by warps even if the tile is not cut
+  constexpr bool     PACKED = !FOLDS;  // (with folds, register pairs spill)
   constexpr uint32_t PARTS = parts(FOLDS);  // partial stages
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1392,7 +1431,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
   pdl_wait();
 
   if (warp < 4) {
-    setmaxnreg_dec<regs_ctrl(FOLDS)>();
+    setmaxnreg_dec<REGS_CTRL>();
     if (warp == 0) {
       // ---------------------------------------------------- TMA producer --
       if (elect_one()) {
@@ -1458,7 +1497,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
     }
   }
   else {
-    setmaxnreg_inc<regs_promo(FOLDS)>();
+    setmaxnreg_inc<REGS_PROMO>();
     // ------------------------------------------- promotion + epilogue ----
     const int      quarter      = warp & 3;         // tensor-memory lane quarter this warp may read
     const int      half         = (warp - 4) >> 2;  // which 64 columns of the scale group
@@ -1515,7 +1554,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
         for (; sc_addr != sc_end; sc_addr += SC_ROW * 4) {
           const uint32_t p = FOLDS ? p3 : it & 3;
           // one fp32 rounding of the scale product, as in the reference
-          float sc = __fmul_rn(lds_f32(sc_addr), lds_f32(sc_addr + sc_b));
+          auto scp = scale_operand<PACKED>(__fmul_rn(lds_f32(sc_addr), lds_f32(sc_addr + sc_b)));
           mbar_wait_at(bars_at + (uint32_t)offsetof(Fp8Pair128Bars, done) + st * 8, st_ph, DEV_WAIT_TMEM_FULL, abort_at, status);
           tc_fence_after_sync();
           uint32_t v0[32], v1[32];
@@ -1527,14 +1566,20 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
           if (lane == 0) {
             mbar_arrive_cluster_relaxed(empty_leader + p * 8);
           }
-          asm volatile("" : "+f"(sc));  // the arithmetic stays behind the hand-back
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            ffma2(acc[i], acc[i + 1], v0[i], v0[i + 1], sc);
+          // the arithmetic stays behind the hand-back
+          if constexpr (PACKED) {
+            asm volatile("" : "+l"(scp));
+          }
+          else {
+            asm volatile("" : "+f"(scp));
           }
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
-            ffma2(acc[32 + i], acc[32 + i + 1], v1[i], v1[i + 1], sc);
+            ffma2(acc[i], acc[i + 1], v0[i], v0[i + 1], scp);
+          }
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            ffma2(acc[32 + i], acc[32 + i + 1], v1[i], v1[i + 1], scp);
           }
           ++it;
           p3 = p3 == 2 ? 0 : p3 + 1;
@@ -1731,7 +1776,7 @@ static int launch_fp8_pair_epi(const void*       A,
   using namespace fp8pair;
   CUtensorMap tm_a, tm_b;
   if (!make_tmap_2d(&tm_a, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)M, (uint64_t)K, BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)
-      || !make_tmap_2d(&tm_b, B, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)N, (uint64_t)K, BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)) {
+      || !make_tmap_2d(&tm_b, B, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)N, (uint64_t)K, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B)) {
     return LLMMM_ERR_CUDA;
   }
   CUtensorMap tm_c = {};
@@ -1963,7 +2008,7 @@ static int launch_fp8_gather(const void*       A,
   }
   CUtensorMap tm_a, tm_b;
   if (!make_tmap_2d(&tm_a, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)M, (uint64_t)K, BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)
-      || !make_tmap_2d(&tm_b, B, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)N, (uint64_t)K, BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)) {
+      || !make_tmap_2d(&tm_b, B, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)K, (uint64_t)N, (uint64_t)K, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B)) {
     return LLMMM_ERR_CUDA;
   }
   static thread_local bool attr_set[64] = {};
@@ -2118,7 +2163,7 @@ extern "C" void llmmm_profile_trace8()
   long long t[64][8];
   cudaMemcpyFromSymbol(t, llmmm::g_trace8, sizeof(t));
   const long long t0 = t[8][0];
-  printf("K-block: MMA[wait_part free operands issued] PROMO[wait observed released]  (clk relative)\n");
+  printf("K-block: MMA[wait operands half0-free half1-free] PROMO[wait observed released]  (clk relative)\n");
   for (int i = 8; i < 24; ++i) {
     printf("%2d: %6lld %6lld %6lld %6lld | %6lld %6lld %6lld\n", i, t[i][0] - t0, t[i][1] - t0, t[i][2] - t0, t[i][3] - t0,
            t[i][4] - t0, t[i][5] - t0, t[i][6] - t0);
