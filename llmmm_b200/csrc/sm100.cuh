@@ -267,6 +267,12 @@ tma_load_2d_hint(void* dst, const CUtensorMap* m, uint64_t* bar, int x, int y, u
     : "memory");
 }
 
+// The tile goes to L2 only.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int x, int y)
+{
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");
+}
+
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* src, int x, int y)
 {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
