@@ -270,9 +270,9 @@ int llmmm_bind_workspace(void* workspace, size_t workspace_bytes);
 
 /* A promise about the B_t / B_scale_t operands of later FP8 GEMM calls from this process: they are model
  * weights, never written by the kernel that runs immediately before the GEMM on the same stream.  With it
- * (enabled != 0) a decode-sized call (M <= 64) reads its first weight tiles and weight scales while the preceding
- * kernel of the stream is still finishing (programmatic dependent launch; activations, their scales and outputs
- * still wait for that kernel).  An earlier kernel of the stream may write them, this library's weight quantiser and
+ * (enabled != 0) a call reads its first weight tiles (a decode-sized one, M <= 64, its weight scales too) while the
+ * preceding kernel of the stream is still finishing (programmatic dependent launch; activations, their scales and
+ * outputs still wait for that kernel).  An earlier kernel of the stream may write them, this library's weight quantiser and
  * transposes among them, unless it releases its dependents early itself (griddepcontrol.launch_dependents before
  * its last store), as no kernel of this library that writes weights does.  Off by default: then nothing is read
  * before the preceding kernel has completed.  No counterpart in the reference. */

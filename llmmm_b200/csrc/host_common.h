@@ -76,6 +76,9 @@ extern thread_local int t_force_mid;
 int launch_fp8_e4m3(const void* A, const float* A_s, const void* B, const float* B_s, void* C, float* C_s, int M, int N, int K,
                     cudaStream_t stream);
 
+// llmmm_set_static_weights()
+extern std::atomic<int> g_static_weights;
+
 // Set by llmmm_check_status() when it reports a device-side wait that ran out: the decode kernel's flagged
 // partial words (registered scratch / built-in scratch) may then hold leftovers and are cleared before the next use.
 extern std::atomic<int> g_scratch_dirty[64];

@@ -220,8 +220,8 @@ __device__ __forceinline__ void mbar_wait_at(uint32_t bar_addr, uint32_t parity,
 // A kernel launched with cudaLaunchAttributeProgrammaticStreamSerialization may start while its
 // predecessor on the stream is still running; pdl_wait() then blocks until that predecessor has
 // completed and its memory is visible.  Everything a kernel does before pdl_wait() must touch no global
-// memory, but for the decode kernel's reads of weights and weight scales that the caller declared static
-// (llmmm_set_static_weights).  pdl_launch_dependents() lets the NEXT kernel on the stream start its own set-up as
+// memory, but for the FP8 kernels' reads of weights (and the decode kernel's of weight scales) that the caller
+// declared static (llmmm_set_static_weights).  pdl_launch_dependents() lets the NEXT kernel on the stream start its own set-up as
 // soon as every CTA of this grid has executed it (or has exited).  Both are no-ops without the attribute.
 //
 // A kernel executes it before its own pdl_wait(), so the kernel after the next one may start while this one is still
