@@ -5,12 +5,12 @@
 // kernel src/mm/fp16/mm.cuh:10-684, an mma.sync.m16n8k16 + ldmatrix kernel with
 // a 256x256 CTA tile).  Nothing of that kernel's structure is kept:
 //
-//   * persistent grid, one CTA per SM, static round-robin over 128x256 tiles;
+//   * persistent grid, one CTA per SM, static round-robin over tiles of 128 rows and 64, 128 or 256 columns (fp16_plan);
 //   * warp 0 (one lane) streams A (K-major) and B (N-major, read in place from
-//     the row-major [K,N] array: no transpose pass) with TMA into a 4-stage
+//     the row-major [K,N] array: no transpose pass) with TMA into a 4- to 8-stage
 //     ring of 128-byte-swizzled shared-memory tiles, completion on mbarriers;
-//   * warp 1 (one lane) issues tcgen05.mma.kind::f16 (128x256x16) into one of
-//     two 256-column TMEM accumulators and commits ring slots back to the
+//   * warp 1 (one lane) issues tcgen05.mma.kind::f16 (128 x width x 16) into one of
+//     two TMEM accumulators and commits ring slots back to the
 //     producer and finished accumulators to the epilogue;
 //   * warps 4-7 drain an accumulator with tcgen05.ld (each lane owns one
 //     output row), convert to the 16-bit type, stage 32x64 sub-tiles in
@@ -30,32 +30,39 @@ namespace llmmm {
 
 namespace fp16cfg {
 constexpr int      BM          = 128;
-constexpr int      BN          = 256;
 constexpr int      BK          = 64;  // 64 x 2 B = one 128-byte swizzle row of A
 constexpr int      UMMA_K      = 16;
-constexpr int      STAGES      = 4;
+constexpr int      MAX_STAGES  = 8;
 constexpr int      THREADS     = 256;
-constexpr uint32_t A_BYTES     = BM * BK * 2;         // 16 KB
-constexpr uint32_t B_BOX_BYTES = 64 * BK * 2;         // one 64(n) x 64(k) box: 8 KB
-constexpr uint32_t B_BYTES     = B_BOX_BYTES * (BN / 64);  // 32 KB
-constexpr uint32_t STAGE_TX    = A_BYTES + B_BYTES;
-constexpr uint32_t C_WARP_BUF  = 32 * 128;  // 32 rows x 64 halves
-constexpr uint32_t OFF_A       = 0;
-constexpr uint32_t OFF_B       = OFF_A + STAGES * A_BYTES;
-constexpr uint32_t OFF_C       = OFF_B + STAGES * B_BYTES;
-constexpr uint32_t OFF_BAR     = OFF_C + 4 * 2 * C_WARP_BUF;
-constexpr uint32_t SMEM_BYTES  = OFF_BAR + 256 + 1024;  // + barrier block + alignment slack
-constexpr uint32_t TMEM_COLS   = 512;                   // two 256-column accumulators
+constexpr uint32_t A_BYTES     = BM * BK * 2;   // 16 KB
+constexpr uint32_t B_BOX_BYTES = 64 * BK * 2;   // one 64(n) x 64(k) box: 8 KB
+constexpr uint32_t C_WARP_BUF  = 32 * 128;      // 32 rows x 64 halves
 }  // namespace fp16cfg
 
+// Shared and tensor memory of the kernel with 128 x BN tiles.
+template<int BN>
+struct Fp16Layout {
+  static constexpr int      STAGES     = BN == 256 ? 4 : BN == 128 ? 6 : 8;
+  static constexpr uint32_t B_BYTES    = fp16cfg::B_BOX_BYTES * (BN / 64);
+  static constexpr uint32_t STAGE_TX   = fp16cfg::A_BYTES + B_BYTES;
+  static constexpr uint32_t OFF_A      = 0;
+  static constexpr uint32_t OFF_B      = OFF_A + STAGES * fp16cfg::A_BYTES;
+  static constexpr uint32_t OFF_C      = OFF_B + STAGES * B_BYTES;
+  static constexpr uint32_t OFF_BAR    = OFF_C + 4 * 2 * fp16cfg::C_WARP_BUF;
+  static constexpr uint32_t SMEM_BYTES = OFF_BAR + 256 + 1024;  // + barrier block + alignment slack
+  static constexpr uint32_t TMEM_COLS  = 2 * BN;                // two accumulators
+  static_assert(STAGES <= fp16cfg::MAX_STAGES && SMEM_BYTES <= 232448, "shared memory of an SM");
+};
+
 struct Fp16Bars {
-  uint64_t full[fp16cfg::STAGES];
-  uint64_t empty[fp16cfg::STAGES];
+  uint64_t full[fp16cfg::MAX_STAGES];
+  uint64_t empty[fp16cfg::MAX_STAGES];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
   uint32_t abort_flag;
 };
+static_assert(sizeof(Fp16Bars) <= 256, "barrier block");
 
 template<typename T>
 __device__ __forceinline__ uint32_t pack2(float a, float b);
@@ -74,16 +81,29 @@ __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b)
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-template<typename T>
+// SPLIT (BN = 64): a tile's K range is cut into `ways` chunks of `chunk` k-steps, one per CTA: CTA c takes chunk c % ways of
+// tile c / ways.  A warp publishes its 32 x 64 fp32 piece of the partial tile (512 contiguous bytes per instruction) and
+// counts its arrival; the warp whose arrival is the last adds the pieces in K order and writes the tile.  Nothing waits
+// for another CTA, the counters are zero again afterwards.
+template<typename T, int BN, bool SPLIT>
 __global__ void __launch_bounds__(fp16cfg::THREADS, 1) fp16_gemm_kernel(const __grid_constant__ CUtensorMap tm_a,
                                                                         const __grid_constant__ CUtensorMap tm_b,
                                                                         const __grid_constant__ CUtensorMap tm_c,
                                                                         int                                 M,
                                                                         int                                 N,
                                                                         int                                 K,
+                                                                        int                                 ways,
+                                                                        int                                 chunk,
+                                                                        float* __restrict__                 partials,
+                                                                        uint32_t* __restrict__              counters,
                                                                         uint32_t*                           status)
 {
   using namespace fp16cfg;
+  using L = Fp16Layout<BN>;
+  static_assert(!SPLIT || BN == 64, "a warp's piece of a cut tile is 32 x 64");
+  constexpr int      STAGES  = L::STAGES;
+  constexpr uint32_t B_BYTES = L::B_BYTES, STAGE_TX = L::STAGE_TX, TMEM_COLS = L::TMEM_COLS;
+  constexpr uint32_t OFF_A = L::OFF_A, OFF_B = L::OFF_B, OFF_C = L::OFF_C, OFF_BAR = L::OFF_BAR;
   extern __shared__ uint8_t smem_raw[];
   uint8_t*  smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   Fp16Bars* bars = reinterpret_cast<Fp16Bars*>(smem + OFF_BAR);
@@ -95,7 +115,11 @@ __global__ void __launch_bounds__(fp16cfg::THREADS, 1) fp16_gemm_kernel(const __
   const int m_tiles   = (M + BM - 1) / BM;
   const int n_tiles   = (N + BN - 1) / BN;
   const int num_tiles = m_tiles * n_tiles;
-  const int k_iters   = (K + BK - 1) / BK;
+  const int k_steps   = (K + BK - 1) / BK;
+  const int first     = SPLIT ? (int)blockIdx.x / ways : (int)blockIdx.x;  // this CTA's first tile
+  const int step      = SPLIT ? num_tiles : (int)gridDim.x;
+  const int k_begin   = SPLIT ? ((int)blockIdx.x % ways) * chunk : 0;
+  const int k_end     = SPLIT ? min(k_begin + chunk, k_steps) : k_steps;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -127,10 +151,10 @@ __global__ void __launch_bounds__(fp16cfg::THREADS, 1) fp16_gemm_kernel(const __
     // ------------------------------------------------------ TMA producer --
     if (elect_one()) {
       uint32_t it = 0;
-      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      for (int tile = first; tile < num_tiles; tile += step) {
         const int m0 = (tile % m_tiles) * BM;
         const int n0 = (tile / m_tiles) * BN;
-        for (int kb = 0; kb < k_iters; ++kb, ++it) {
+        for (int kb = k_begin; kb < k_end; ++kb, ++it) {
           const uint32_t s  = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           mbar_wait(&bars->empty[s], ph ^ 1, DEV_WAIT_SMEM_EMPTY, abort_flag, status);
@@ -151,13 +175,13 @@ __global__ void __launch_bounds__(fp16cfg::THREADS, 1) fp16_gemm_kernel(const __
       constexpr uint32_t idesc = make_idesc(kFmt, kFmt, /*a_mn=*/0, /*b_mn=*/1, BM, BN);
       uint32_t           it    = 0;
       uint32_t           t     = 0;
-      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++t) {
+      for (int tile = first; tile < num_tiles; tile += step, ++t) {
         const uint32_t acc    = t & 1;
         const uint32_t acc_ph = (t >> 1) & 1;
         mbar_wait(&bars->tmem_empty[acc], acc_ph ^ 1, DEV_WAIT_TMEM_EMPTY, abort_flag, status);
         tc_fence_after_sync();
         const uint32_t d_addr = tmem_base + acc * BN;
-        for (int kb = 0; kb < k_iters; ++kb, ++it) {
+        for (int kb = k_begin; kb < k_end; ++kb, ++it) {
           const uint32_t s  = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           mbar_wait(&bars->full[s], ph, DEV_WAIT_SMEM_FULL, abort_flag, status);
@@ -171,7 +195,7 @@ __global__ void __launch_bounds__(fp16cfg::THREADS, 1) fp16_gemm_kernel(const __
                        da + (uint64_t)((kk * UMMA_K * 2) >> 4),
                        db + (uint64_t)((kk * UMMA_K * 128) >> 4),
                        idesc,
-                       (kb | kk) != 0);
+                       ((kb - k_begin) | kk) != 0);
           }
           tc_commit(&bars->empty[s]);
         }
@@ -185,7 +209,7 @@ __global__ void __launch_bounds__(fp16cfg::THREADS, 1) fp16_gemm_kernel(const __
     uint8_t*       cbuf     = smem + OFF_C + ew * 2 * C_WARP_BUF;
     uint32_t       t        = 0;
     uint32_t       chunk_it = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++t) {
+    for (int tile = first; tile < num_tiles; tile += step, ++t) {
       const int      m0     = (tile % m_tiles) * BM;
       const int      n0     = (tile / m_tiles) * BN;
       const uint32_t acc    = t & 1;
@@ -205,6 +229,46 @@ __global__ void __launch_bounds__(fp16cfg::THREADS, 1) fp16_gemm_kernel(const __
           __syncwarp();
           if (lane == 0) {
             mbar_arrive(&bars->tmem_empty[acc]);
+          }
+        }
+        if constexpr (SPLIT) {
+          // [CTA][warp][16 pieces of 4 columns][lane]
+          float4* mine = reinterpret_cast<float4*>(partials) + ((size_t)blockIdx.x * 4 + ew) * 512 + lane;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            __stcg(mine + j * 32, make_float4(__uint_as_float(v0[4 * j]), __uint_as_float(v0[4 * j + 1]), __uint_as_float(v0[4 * j + 2]), __uint_as_float(v0[4 * j + 3])));
+            __stcg(mine + (8 + j) * 32, make_float4(__uint_as_float(v1[4 * j]), __uint_as_float(v1[4 * j + 1]), __uint_as_float(v1[4 * j + 2]), __uint_as_float(v1[4 * j + 3])));
+          }
+          __threadfence();
+          __syncwarp();
+          uint32_t arrived = 0;
+          if (lane == 0) {
+            arrived = atomicAdd(&counters[tile * 4 + ew], 1u);
+          }
+          arrived = __shfl_sync(0xffffffffu, arrived, 0);
+          if (arrived != (uint32_t)(ways - 1)) {
+            continue;  // another warp finishes this piece
+          }
+          __threadfence();
+          for (int w = 0; w < ways; ++w) {  // in K order: the result does not depend on timing
+            const float4* src = reinterpret_cast<const float4*>(partials) + ((size_t)(tile * ways + w) * 4 + ew) * 512 + lane;
+            float4        t[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              t[j] = __ldcg(src + j * 32);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float a[8] = {t[j].x, t[j].y, t[j].z, t[j].w, t[8 + j].x, t[8 + j].y, t[8 + j].z, t[8 + j].w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                v0[4 * j + e] = __float_as_uint(w == 0 ? a[e] : __uint_as_float(v0[4 * j + e]) + a[e]);
+                v1[4 * j + e] = __float_as_uint(w == 0 ? a[4 + e] : __uint_as_float(v1[4 * j + e]) + a[4 + e]);
+              }
+            }
+          }
+          if (lane == 0) {
+            counters[tile * 4 + ew] = 0;  // every launch leaves the counters at zero
           }
         }
         uint8_t* buf = cbuf + (chunk_it & 1) * C_WARP_BUF;
@@ -672,17 +736,11 @@ __global__ void __launch_bounds__(fp16pair::THREADS, 1)
 }
 
 template<typename T>
-static int launch_fp16_pair(const void* A, const void* B, void* C, int M, int N, int K, const DeviceInfo* info, cudaStream_t stream)
+static int launch_fp16_pair(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_c, int M, int N, int K,
+                            const SplitPlan& plan, const DeviceInfo* info, cudaStream_t stream)
 {
   using namespace fp16pair;
-  constexpr CUtensorMapDataType dt =
-    std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  CUtensorMap tm_a, tm_b, tm_c;
-  if (!make_tmap_2d(&tm_a, A, dt, 2, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, 128, CU_TENSOR_MAP_SWIZZLE_128B)
-      || !make_tmap_2d(&tm_b, B, dt, 2, (uint64_t)N, (uint64_t)K, (uint64_t)N * 2, 64, BK, CU_TENSOR_MAP_SWIZZLE_128B)
-      || !make_tmap_2d(&tm_c, C, dt, 2, (uint64_t)N, (uint64_t)M, (uint64_t)N * 2, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B)) {
-    return LLMMM_ERR_CUDA;
-  }
+  static_assert(BK == fp16cfg::BK, "both kernels take the same tensor maps");
   static thread_local bool attr_set[64] = {};
   if (!attr_set[info->device]) {
     LLMMM_CUDA_TRY(
@@ -691,10 +749,6 @@ static int launch_fp16_pair(const void* A, const void* B, void* C, int M, int N,
       cudaFuncSetAttribute(fp16_gemm_pair_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
     attr_set[info->device] = true;
   }
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  // estimated cost of a split, in K-steps of 64 (one takes about 0.33 us): publishing a chunk and counting
-  // the arrival about 3 us, reading a chunk back about 1.5 us
-  const SplitPlan plan = plan_split(info, tiles, (K + BK - 1) / BK, /*fixed*/ 10, /*per_way_x2*/ 9, /*min_gain*/ 6);
   if (plan.split_pairs > 0) {
     LLMMM_CUDA_TRY(launch_pdl(fp16_gemm_pair_kernel<T, true>, dim3(2 * plan.pairs), dim3(THREADS), SMEM_BYTES, stream, 2, tm_a,
                               tm_b, tm_c, M, N, K, plan.dp_tiles, plan.split_pairs, plan.split_s, plan.split_chunk,
@@ -709,30 +763,90 @@ static int launch_fp16_pair(const void* A, const void* B, void* C, int M, int N,
   return LLMMM_OK;
 }
 
-// Which kernel a problem runs on: more than 128 rows (and columns) the pair kernel; 65..128 rows the single-CTA
-// kernel, unless its tiles would occupy at most half of the SMs and scratch is registered: then the pair
-// kernel, whose tiles can be cut along K (the same rule as for FP8).
-static bool fp16_use_pair_kernel(const DeviceInfo* info, int M, int N)
+// Which kernel a problem runs on.
+struct Fp16Plan {
+  bool      pair;   // 256x256 tiles, cut along K as `split` says
+  SplitPlan split;
+  int       bn;     // else: width of the single-CTA kernel's tiles,
+  int       ways;   // the chunks a tile is cut into along K,
+  int       chunk;  // and k-steps per chunk
+};
+
+// Times in ns, from a sweep of 19 shapes as launch chains (256..1333 x 256..4096 x 256..9728 and 1..128 rows): a pair kernel
+// takes 5400 and 280 per k-step of 64 and round of tiles, the single-CTA kernel 2900 and 153 / 200 / 270 per k-step for tiles
+// 64 / 128 / 256 wide.  A k-step of a 128x64 tile is 128 clk of MMAs, but 24 KB that one SM has to fetch.  Problems of one wave
+// took the pair kernel (cut along K if they were long) before they took narrow tiles: 256^3 5.5 -> 2.9 us, 512x1024x1024 9.0 ->
+// 4.7, 1001x1024x1544 11.9 -> 8.2, 512x2048x4096 22.8 -> 12.7; with the narrow tiles cut along K 256x256x4096 19.6 -> 8.7 (10.8
+// not cut), 300x1288x3592 21.7 -> 13.6; of up to 128 rows 16x4096x4096 22.5 -> 12.5, 128x12288x1024 10.7 -> 8.0.
+static Fp16Plan fp16_plan(const DeviceInfo* info, int M, int N, int K, bool count)
 {
-  if (info->max_pairs < 1 || N <= 128) {
-    return false;
+  const int       k_steps = (K + fp16cfg::BK - 1) / fp16cfg::BK;
+  const int       m_tiles = (M + fp16cfg::BM - 1) / fp16cfg::BM;
+  const Workspace ws      = registered_workspace(info->device);
+  const bool      scratch = ws.ptr != nullptr && ws.bytes >= split_workspace_bytes();
+  auto            tiles   = [&](int bn) { return m_tiles * ((N + bn - 1) / bn); };
+  const int       tiles_pair = ((M + 255) / 256) * ((N + 255) / 256);
+  // estimated cost of a split, in k-steps: publishing a chunk and counting the arrival about 3 us, reading a chunk back
+  // about 1.5 us
+  auto pair_plan = [&](bool c) { return plan_split(info, tiles_pair, k_steps, /*fixed*/ 10, /*per_way_x2*/ 9, /*min_gain*/ 6, c); };
+
+  // The narrowest tiles that are still one wave: as many SMs as possible fetch operands (128x4096x4096 26.0 us with tiles 256
+  // wide, 16.3 with 128, 12.9 with 64; 64x12288x4096, where 64 wide is two waves, 27.8, 19.7, 25.3).
+  Fp16Plan plan{};
+  plan.ways  = 1;
+  plan.chunk = k_steps;
+  plan.bn    = tiles(64) <= info->sm_count ? 64 : tiles(128) <= info->sm_count ? 128 : 256;
+  if (info->max_pairs < 1 || N <= 128 || M <= 64) {
+    return plan;  // (calls of up to 64 rows never use scratch)
   }
-  if (M > 128) {
-    return true;
+  if (M <= 128) {
+    // 65..128 rows: the pair kernel if it cuts its few tiles along K
+    const SplitPlan sp = scratch && 2 * tiles(256) <= info->sm_count ? pair_plan(false) : SplitPlan{};
+    plan.pair          = sp.split_pairs > 0;
+    if (plan.pair) {
+      plan.split = pair_plan(count);
+    }
+    return plan;
   }
-  const int       tiles_1cta = ((M + fp16cfg::BM - 1) / fp16cfg::BM) * ((N + fp16cfg::BN - 1) / fp16cfg::BN);
-  const Workspace ws         = registered_workspace(info->device);
-  return M > 64 && ws.ptr != nullptr && ws.bytes >= split_workspace_bytes() && 2 * tiles_1cta <= info->sm_count;
+  long long narrow = -1;
+  if (plan.bn < 256) {
+    narrow = 2900 + (plan.bn == 64 ? 153ll : 200ll) * k_steps;
+    if (plan.bn == 64 && scratch) {
+      const int max_ways = info->sm_count / tiles(64) < SPLIT_MAX_WAYS ? info->sm_count / tiles(64) : SPLIT_MAX_WAYS;
+      for (int w = 2; w <= max_ways; ++w) {
+        const int       c   = (k_steps + w - 1) / w;
+        const long long est = 2900 + 153ll * c + 2000 + 300 * w;
+        if (est < narrow) {
+          narrow     = est;
+          plan.chunk = c;
+          plan.ways  = (k_steps + c - 1) / c;  // no empty chunks
+        }
+      }
+    }
+  }
+  const SplitPlan sp     = pair_plan(false);
+  const long long rounds = sp.dp_tiles > 0 ? (sp.dp_tiles + sp.pairs - 1) / sp.pairs : 0;
+  const long long pair   = 5400 + 280 * (rounds * k_steps + (sp.split_pairs > 0 ? sp.split_chunk : 0))
+                         + (sp.split_pairs > 0 ? 3000 + 1500 * sp.split_s : 0);
+  plan.pair = narrow < 0 || pair < narrow;
+  if (plan.pair) {
+    plan.split = pair_plan(count);
+  }
+  else if (plan.ways > 1 && count) {
+    g_split_launches.fetch_add(1);
+  }
+  return plan;
 }
 
 void describe_fp16_plan(const DeviceInfo* info, bool bf16, int M, int N, int K, char* buf, size_t len)
 {
   const char* t = bf16 ? "__nv_bfloat16" : "__half";
-  if (fp16_use_pair_kernel(info, M, N)) {
+  const Fp16Plan chosen = fp16_plan(info, M, N, K, false);
+  if (chosen.pair) {
     using namespace fp16pair;
-    const int       tiles   = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-    const int       k_steps = (K + BK - 1) / BK;
-    const SplitPlan plan    = plan_split(info, tiles, k_steps, 10, 9, 6, false);
+    const int        tiles   = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+    const int        k_steps = (K + BK - 1) / BK;
+    const SplitPlan& plan    = chosen.split;
     if (plan.split_pairs > 0) {
       snprintf(buf, len, "fp16_gemm_pair_kernel<%s>: %d tiles of 256x256 on %d CTA pairs; %d whole tiles round-robin, then %d "
                "tiles cut %d-way along K (chunks of %d k-steps of 64), one chunk per pair", t, tiles, plan.pairs, plan.dp_tiles,
@@ -744,10 +858,15 @@ void describe_fp16_plan(const DeviceInfo* info, bool bf16, int M, int N, int K, 
     }
     return;
   }
-  using namespace fp16cfg;
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  const int grid  = tiles < info->sm_count ? tiles : info->sm_count;
-  snprintf(buf, len, "fp16_gemm_kernel<%s>: %d tiles of %dx%d on %d CTAs (%.2f waves)", t, tiles, BM, BN, grid, (double)tiles / grid);
+  const int bn    = chosen.bn;
+  const int tiles = ((M + fp16cfg::BM - 1) / fp16cfg::BM) * ((N + bn - 1) / bn);
+  if (chosen.ways > 1) {
+    snprintf(buf, len, "fp16_gemm_kernel<%s>: %d tiles of %dx%d cut %d-way along K (chunks of %d k-steps of 64), one chunk per CTA", t, tiles,
+             fp16cfg::BM, bn, chosen.ways, chosen.chunk);
+    return;
+  }
+  const int grid = tiles < info->sm_count ? tiles : info->sm_count;
+  snprintf(buf, len, "fp16_gemm_kernel<%s>: %d tiles of %dx%d on %d CTAs (%.2f waves)", t, tiles, fp16cfg::BM, bn, grid, (double)tiles / grid);
 }
 
 int warm_fp16_kernels(const DeviceInfo* info)
@@ -757,8 +876,33 @@ int warm_fp16_kernels(const DeviceInfo* info)
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp16_gemm_pair_kernel<__half, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp16pair::SMEM_BYTES));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp16_gemm_pair_kernel<__nv_bfloat16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp16pair::SMEM_BYTES));
   LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp16_gemm_pair_kernel<__nv_bfloat16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp16pair::SMEM_BYTES));
-  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp16_gemm_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp16cfg::SMEM_BYTES));
-  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp16_gemm_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp16cfg::SMEM_BYTES));
+#define LLMMM_WARM_FP16(T, BN, SPLIT)                                                                                  \
+  LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp16_gemm_kernel<T, BN, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Fp16Layout<BN>::SMEM_BYTES));
+  LLMMM_WARM_FP16(__half, 64, false) LLMMM_WARM_FP16(__half, 64, true) LLMMM_WARM_FP16(__half, 128, false) LLMMM_WARM_FP16(__half, 256, false)
+  LLMMM_WARM_FP16(__nv_bfloat16, 64, false) LLMMM_WARM_FP16(__nv_bfloat16, 64, true) LLMMM_WARM_FP16(__nv_bfloat16, 128, false)
+  LLMMM_WARM_FP16(__nv_bfloat16, 256, false)
+#undef LLMMM_WARM_FP16
+  return LLMMM_OK;
+}
+
+template<typename T, int BN, bool SPLIT>
+static int launch_fp16_1cta(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_c, int M, int N, int K,
+                            const Fp16Plan& plan, const DeviceInfo* info, cudaStream_t stream)
+{
+  using namespace fp16cfg;
+  static thread_local bool attr_set[64] = {};
+  if (!attr_set[info->device]) {
+    LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp16_gemm_kernel<T, BN, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Fp16Layout<BN>::SMEM_BYTES));
+    attr_set[info->device] = true;
+  }
+  const int tiles    = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  const int grid     = SPLIT ? tiles * plan.ways : (tiles < info->sm_count ? tiles : info->sm_count);
+  uint8_t*  ws       = SPLIT ? static_cast<uint8_t*>(registered_workspace(info->device).ptr) : nullptr;
+  float*    partials = SPLIT ? reinterpret_cast<float*>(ws + WS_HEADER_BYTES) : nullptr;
+  uint32_t* counters = SPLIT ? reinterpret_cast<uint32_t*>(ws + WS_RESERVED_BYTES) : nullptr;
+  LLMMM_CUDA_TRY(launch_pdl(fp16_gemm_kernel<T, BN, SPLIT>, dim3(grid), dim3(THREADS), Fp16Layout<BN>::SMEM_BYTES, stream, 1, tm_a, tm_b,
+                            tm_c, M, N, K, plan.ways, plan.chunk, partials, counters, info->status));
+  g_launches.fetch_add(1);
   return LLMMM_OK;
 }
 
@@ -787,23 +931,18 @@ static int launch_fp16(const void* A, const void* B, void* C, int M, int N, int 
       || !make_tmap_2d(&tm_c, C, dt, 2, (uint64_t)N, (uint64_t)M, (uint64_t)N * 2, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B)) {
     return LLMMM_ERR_CUDA;
   }
-  if (fp16_use_pair_kernel(info, M, N)) {
-    return launch_fp16_pair<T>(A, B, C, M, N, K, info, stream);
+  const Fp16Plan plan = fp16_plan(info, M, N, K, true);
+  if (plan.pair) {
+    return launch_fp16_pair<T>(tm_a, tm_b, tm_c, M, N, K, plan.split, info, stream);
   }
-  static thread_local bool attr_set[64] = {};
-  if (!attr_set[info->device]) {
-    LLMMM_CUDA_TRY(
-      cudaFuncSetAttribute(fp16_gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
-    attr_set[info->device] = true;
+  if (plan.ways > 1) {
+    return launch_fp16_1cta<T, 64, true>(tm_a, tm_b, tm_c, M, N, K, plan, info, stream);
   }
-  const int m_tiles = (M + BM - 1) / BM;
-  const int n_tiles = (N + BN - 1) / BN;
-  const int tiles   = m_tiles * n_tiles;
-  const int grid    = tiles < info->sm_count ? tiles : info->sm_count;
-  LLMMM_CUDA_TRY(launch_pdl(fp16_gemm_kernel<T>, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, 1, tm_a, tm_b, tm_c, M, N, K,
-                            info->status));
-  g_launches.fetch_add(1);
-  return LLMMM_OK;
+  switch (plan.bn) {
+    case 64: return launch_fp16_1cta<T, 64, false>(tm_a, tm_b, tm_c, M, N, K, plan, info, stream);
+    case 128: return launch_fp16_1cta<T, 128, false>(tm_a, tm_b, tm_c, M, N, K, plan, info, stream);
+    default: return launch_fp16_1cta<T, 256, false>(tm_a, tm_b, tm_c, M, N, K, plan, info, stream);
+  }
 }
 
 }  // namespace llmmm

@@ -173,3 +173,28 @@ def test_other_stream(capi, oracle, cuda):
     s.synchronize()
     exact = oracle.exact_gemm(dA.float().cpu().numpy(), dB.float().cpu().numpy())
     assert np.abs(dC.float().cpu().numpy() - exact).max() <= 2e-3 * np.abs(exact).max()
+
+
+# (M, N, K, tile width, ways along K with scratch): one wave of 128-row tiles.  Edges of a tile, ragged last tiles and k-steps,
+# the most tiles of either width on 148 SMs, a last chunk along K that is shorter than the others.
+NARROW_SHAPES = [(129, 136, 72, 64, 1), (256, 1160, 1544, 64, 1), (64, 9472, 64, 64, 1), (33, 9480, 200, 128, 1), (130, 9472, 72, 128, 1),
+                 (256, 256, 4096, 64, 6), (130, 1096, 4104, 64, 4), (385, 1096, 3592, 64, 2)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shape", NARROW_SHAPES, ids=lambda s: "x".join(map(str, s[:3])))
+def test_one_wave_of_narrow_tiles(capi, oracle, cuda, shape, dtype):
+    M, N, K, width, ways = shape
+    if torch.cuda.get_device_properties(cuda).multi_processor_count != 148:
+        pytest.skip("the tile width follows the number of SMs")
+    capi.clear_workspace()
+    d = capi.describe_plan("fp16", M, N, K)
+    assert f"tiles of 128x{width}" in d and "cut" not in d
+    run_case(capi, oracle, cuda, M, N, K, dtype, seed=9, scratch=False)
+    capi.ensure_workspace(M, max(N, 128), max(K, 128))
+    d = capi.describe_plan("fp16", M, N, K)
+    assert f"tiles of 128x{width}" in d and (f"cut {ways}-way" in d if ways > 1 else "cut" not in d)
+    n0 = capi.split_launch_count()
+    for _ in range(2):  # (the second call finds the arrival counters as the first one left them)
+        run_case(capi, oracle, cuda, M, N, K, dtype, seed=9, scratch=True)
+    assert capi.split_launch_count() == n0 + (2 if ways > 1 else 0)
