@@ -213,8 +213,9 @@ int llmmm_transpose_aligned_128(void* dst, const void* src, int M, int N, int el
  * current device.  Two paths use it: the decode-sized (M <= 64) FP8 kernel and
  * hooks, and, for M > 128 (FP16/BF16: M > 64), the kernels with 256x256 tiles
  * when their last wave would leave most of the GPU idle, and the FP16/BF16 kernel
- * with 128x64 tiles when those are few (M > 128): the tiles are then cut along K, the fp32 partial tiles go through the scratch and are added in a
- * fixed order (results are bitwise stable from call to call, and differ from the
+ * with 128x64 tiles when those are few (M > 128): the tiles are then cut along
+ * K, the fp32 partial tiles go through the scratch and are added in a fixed
+ * order (results are bitwise stable from call to call, and differ from the
  * unsplit ones only by the association of fp32 sums).  With scratch registered,
  * FP8 problems of M > 64 with few tiles run on 128x256 tiles instead, cut along K
  * on chip; such a call leaves the scratch alone.  llmmm_fp8_workspace_bytes gives
