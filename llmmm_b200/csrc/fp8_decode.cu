@@ -16,11 +16,9 @@
 //     groups, and only the left-over groups are cut evenly among the CTAs,
 //     which work on those cut pieces FIRST;
 //   * warp 0 streams weight blocks (and the matching activation slab) through
-//     a 6-8-deep TMA ring; warps 1-3 take turns issuing the MMAs of a K-block
-//     (four per K-block, from zero, into the tensor-memory partial stage of the
-//     ring slot): a thread that issues four MMAs and a commit is held for about
-//     640 clk whatever their width, so one thread alone could not keep up with
-//     the ring; the promotion warps (4, or 8 for 32 and 64 columns) promote
+//     a 6-8-deep TMA ring; warp 1 (32 and 64 columns: warps 1-3 in turn) issues
+//     the MMAs of a K-block (four per K-block, from zero, into the tensor-memory
+//     partial stage of the ring slot); the promotion warps (4, or 8 for 32 and 64 columns) promote
 //     with acc = fma(partial, A_s*B_s, acc) in registers, the scale products of
 //     a whole run staged through shared memory ahead of time (a load per
 //     K-block would put an L2 round trip into every iteration);
@@ -54,7 +52,7 @@ namespace deccfg {
 constexpr int      BK            = 128;
 constexpr int      UMMA_K        = 32;
 constexpr int      MAX_STAGES    = 8;    // the ring depth depends on the activation tile, see DecodeSmem
-// warps 0-3: producer, three MMA issuers; warps 4-7 (up to 16 activation columns) or 4-11 (32, 64 columns): promotion.
+// warps 0-3: producer, one or three MMA issuers; warps 4-7 (up to 16 activation columns) or 4-11 (32, 64 columns): promotion.
 // With 64 columns one promotion warp per scheduler could not keep up with the weight stream (measured: ~600 ns per
 // K-block, all of it latency: shared-memory loads, the barrier, tensor-memory loads, 64 FMAs, one after the other
 // with nothing to overlap; HBM delivers a block every 364 ns): two warps per scheduler take half of the columns
@@ -105,7 +103,7 @@ struct DecodeSmem {
   static constexpr int      STAGES     = MP <= 16 ? 6 : 8;
   // K-block `it` uses ring stage it % STAGES and the tensor-memory partial stage of the same index, so ONE
   // tcgen05.commit per K-block tells both the promotion warps (partial ready) and the producer (operands
-  // consumed); a second commit would cost the single issuing thread another ~150 clk per K-block.
+  // consumed).
   static constexpr uint32_t PART_COLS  = MP < 32 ? 32 : MP;
   static constexpr uint32_t TMEM_COLS  = STAGES * PART_COLS <= 256 ? 256 : 512;  // one partial stage per ring stage
   static_assert(STAGES * PART_COLS <= TMEM_COLS, "partial stages exceed the tensor memory allocation");
@@ -173,6 +171,21 @@ __device__ __forceinline__ void epilogue_bar_sync()
 __device__ __forceinline__ int cta_of_unit(uint32_t u, uint32_t G, uint32_t U)
 {
   return (int)(((u + 1) * G - 1) / U);
+}
+
+// d{0,1} = fma(a{0,1}, s{0,1}, d{0,1}) as one packed instruction, the same two roundings (half the issue slots).
+__device__ __forceinline__ void fma_pair(float& d0, float& d1, uint32_t a0, uint32_t a1, float s0, float s1)
+{
+  asm("{\n\t"
+      ".reg .b64 d, a, s;\n\t"
+      "mov.b64 d, {%0, %1};\n\t"
+      "mov.b64 a, {%2, %3};\n\t"
+      "mov.b64 s, {%4, %5};\n\t"
+      "fma.rn.f32x2 d, a, s, d;\n\t"
+      "mov.b64 {%0, %1}, d;\n\t"
+      "}"
+      : "+f"(d0), "+f"(d1)
+      : "r"(a0), "r"(a1), "f"(s0), "f"(s1));
 }
 
 // One output group that was cut among several CTAs, as seen by one promotion warp of a contributor.
@@ -663,12 +676,15 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
     }
   }
   else if (warp < EPI_WARP0) {
-    // --------------------------------------------- three MMA issuers ------
-    // Warps 1, 2 and 3 take every third K-block of the run; each K-block has its own ring slot and
-    // tensor-memory partial stage, so the threads never touch the same barrier phase.
-    if (elect_one()) {
+    // --------------------------------------------- MMA issuers ------------
+    // Up to 16 columns warp 1 alone, else warps 1, 2 and 3 in turn; each K-block has its own ring slot and tensor-memory
+    // partial stage, so the threads never touch the same barrier phase.  (One thread under elect.sync keeps up; with packed
+    // FMAs beside it, layer at M = 1 / 16: 38.45 / 41.2 us with three threads, 38.2 / 40.9 with one; the GEMMs at M = 64
+    // 38.8 and 38.95 as a graph.)
+    constexpr int ISSUERS = MP <= 16 ? 1 : 3;
+    if (warp <= ISSUERS && elect_one()) {
       constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, 128, MP);
-      for (uint32_t it = (uint32_t)(warp - 1); it < run; it += 3) {
+      for (uint32_t it = (uint32_t)(warp - 1); it < run; it += ISSUERS) {
         const uint32_t s  = it % L::STAGES;
         const uint32_t ph = (it / L::STAGES) & 1;
         mbar_wait(&bars->part_empty[s], ph ^ 1, DEV_WAIT_TMEM_EMPTY, abort_flag, status);
@@ -830,18 +846,14 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
         PROF_KB(2);
 #pragma unroll
         for (int i = 0; i < H4; ++i) {
-          acc[4 * i]     = __fmaf_rn(__uint_as_float(v[4 * i]), s_lo[i].x, acc[4 * i]);
-          acc[4 * i + 1] = __fmaf_rn(__uint_as_float(v[4 * i + 1]), s_lo[i].y, acc[4 * i + 1]);
-          acc[4 * i + 2] = __fmaf_rn(__uint_as_float(v[4 * i + 2]), s_lo[i].z, acc[4 * i + 2]);
-          acc[4 * i + 3] = __fmaf_rn(__uint_as_float(v[4 * i + 3]), s_lo[i].w, acc[4 * i + 3]);
+          fma_pair(acc[4 * i], acc[4 * i + 1], v[4 * i], v[4 * i + 1], s_lo[i].x, s_lo[i].y);
+          fma_pair(acc[4 * i + 2], acc[4 * i + 3], v[4 * i + 2], v[4 * i + 3], s_lo[i].z, s_lo[i].w);
         }
 #pragma unroll
         for (int i = 0; i < H4; ++i) {
           const int m = 4 * (H4 + i);
-          acc[m]     = __fmaf_rn(__uint_as_float(v[m]), s_hi[i].x, acc[m]);
-          acc[m + 1] = __fmaf_rn(__uint_as_float(v[m + 1]), s_hi[i].y, acc[m + 1]);
-          acc[m + 2] = __fmaf_rn(__uint_as_float(v[m + 2]), s_hi[i].z, acc[m + 2]);
-          acc[m + 3] = __fmaf_rn(__uint_as_float(v[m + 3]), s_hi[i].w, acc[m + 3]);
+          fma_pair(acc[m], acc[m + 1], v[m], v[m + 1], s_hi[i].x, s_hi[i].y);
+          fma_pair(acc[m + 2], acc[m + 3], v[m + 2], v[m + 3], s_hi[i].z, s_hi[i].w);
         }
         PROF_KB(3);
       }
