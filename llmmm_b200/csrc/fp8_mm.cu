@@ -43,6 +43,10 @@
 
 namespace llmmm {
 
+// Static weight tiles beyond the ring that the kernels for up to 128 rows request into L2 before the dependency wait: the four
+// GEMMs of a Qwen3-4B layer at 100 rows with none 48.5 us, four 48.6, eight 48.2, twelve and more 48.8.
+constexpr int EARLY_L2 = 8;
+
 namespace fp8cfg {
 constexpr int      BM         = 128;
 constexpr int      BN         = 256;
@@ -220,6 +224,9 @@ __global__ void __launch_bounds__(fp8cfg::THREADS, 1) fp8_blockwise_gemm_kernel(
       for (uint32_t s = 0; s < early; ++s) {
         mbar_arrive_expect_tx(&bars->full[s], STAGE_TX);
         tma_load_2d(smem + OFF_B + s * B_BYTES, &tm_b, &bars->full[s], (int)s * BK, ((int)blockIdx.x / m_tiles) * BN);
+      }
+      for (int kb = (int)early; kb < min((int)early + EARLY_L2, early > 0 ? k_blocks : 0); ++kb) {
+        tma_prefetch_2d(&tm_b, kb * BK, ((int)blockIdx.x / m_tiles) * BN);
       }
     }
     __syncwarp();
@@ -1491,6 +1498,11 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
       if (elect_one()) {
         for (int kb = kb0; kb < early_end; ++kb) {
           load_weights((uint32_t)(kb - kb0), kb);
+        }
+        if (early_weights) {  // (and the EARLY_L2 tiles behind the ring go to L2)
+          for (int kb = early_end; kb < min(early_end + EARLY_L2, kb1); ++kb) {
+            tma_prefetch_2d(&tm_b, kb * BK, SWIGLU ? tile * 128 + (int)rank * N : tile * BN + (int)rank * 128);
+          }
         }
       }
       __syncwarp();
