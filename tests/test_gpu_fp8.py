@@ -297,6 +297,42 @@ def test_static_weights_written_by_the_kernel_before_the_last(capi, cuda, M, NK)
     capi.check_status()
 
 
+# single-CTA, 128-row pair and 256-row pair kernel: K longer than the ring and the tiles requested into L2, K shorter than the
+# ring, an odd number of groups (a second column half beyond the matrix), tiles and slices cut along K
+@pytest.mark.parametrize("shape", [(100, 19456, 2560), (100, 19456, 256), (100, 2560, 9728), (100, 384, 256), (300, 9600, 1920), (2310, 640, 256),
+                                   (2304, 4352, 2048)], ids=lambda s: "x".join(map(str, s)))
+def test_static_weights_above_64_rows(capi, cuda, shape):
+    # the first weight tiles are read before the quantiser of the activations has finished, the activations are not
+    M, N, K = shape
+    g = torch.Generator(device=cuda).manual_seed(65)
+    x = [torch.randn(M, K, device=cuda, generator=g) * s for s in (1.0, 4.0)]
+    w = [torch.randn(N, K, device=cuda, generator=g) * 0.02 for _ in range(2)]
+    A_q, A_s = torch.empty(M, K, dtype=torch.uint8, device=cuda), torch.empty(K // 128, M, device=cuda)
+    B_q, B_s = torch.empty(N, K, dtype=torch.uint8, device=cuda), torch.empty(N // 128, K // 128, device=cuda)
+    C, C_q, C_s = torch.empty(M, N, device=cuda), torch.empty(M, N, dtype=torch.uint8, device=cuda), torch.empty(N // 128, M, device=cuda)
+    capi.ensure_workspace(M, N, K)
+
+    def call(i, wait):
+        capi.fp8_quant_128x128(w[i], B_q, B_s, N, K)
+        wait()
+        capi.fp8_quant_1x128(x[i], A_q, A_s, M, K)
+        capi.fp8_blockwise_mm_f32(A_q, A_s, B_q, B_s, C, M, N, K)
+        capi.fp8_quant_1x128(x[1 - i], A_q, A_s, M, K)
+        capi.fp8_blockwise_mm(A_q, A_s, B_q, B_s, C_q, C_s, M, N, K)
+        return C.clone(), C_q.clone(), C_s.clone()
+
+    capi.set_static_weights(False)
+    expected = [call(i, torch.cuda.synchronize) for i in range(2)]
+    capi.set_static_weights(True)
+    try:
+        for rep in range(6):
+            for a, b in zip(call(rep & 1, lambda: None), expected[rep & 1]):
+                assert torch.equal(a, b)
+    finally:
+        capi.set_static_weights(False)
+    capi.check_status()
+
+
 @pytest.mark.parametrize("shape", [(128, 2560, 4096), (65, 512, 2048), (100, 4096, 1024)])
 def test_mid_m_few_tiles_take_the_pair_kernel_with_scratch(capi, oracle, cuda, shape):
     # 65..128 rows, tiles on at most half of the SMs: single-CTA kernel without scratch, pair kernel (whose tiles
