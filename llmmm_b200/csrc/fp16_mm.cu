@@ -769,7 +769,9 @@ struct Fp16Plan {
   SplitPlan split;
   int       bn;     // else: width of the single-CTA kernel's tiles,
   int       ways;   // the chunks a tile is cut into along K,
-  int       chunk;  // and k-steps per chunk
+  int       chunk;  // k-steps per chunk,
+  float*    partials;  // and, with ways > 1, the scratch that was there when the plan was made
+  uint32_t* counters;
 };
 
 // Times in ns, from a sweep of 19 shapes as launch chains (256..1333 x 256..4096 x 256..9728 and 1..128 rows): a pair kernel
@@ -823,6 +825,11 @@ static Fp16Plan fp16_plan(const DeviceInfo* info, int M, int N, int K, bool coun
         }
       }
     }
+  }
+  if (plan.ways > 1) {
+    // (the launch must not look the scratch up again: another thread may unregister or replace it meanwhile)
+    plan.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(ws.ptr) + WS_HEADER_BYTES);
+    plan.counters = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(ws.ptr) + WS_RESERVED_BYTES);
   }
   const SplitPlan sp     = pair_plan(false);
   const long long rounds = sp.dp_tiles > 0 ? (sp.dp_tiles + sp.pairs - 1) / sp.pairs : 0;
@@ -895,13 +902,10 @@ static int launch_fp16_1cta(const CUtensorMap& tm_a, const CUtensorMap& tm_b, co
     LLMMM_CUDA_TRY(cudaFuncSetAttribute(fp16_gemm_kernel<T, BN, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Fp16Layout<BN>::SMEM_BYTES));
     attr_set[info->device] = true;
   }
-  const int tiles    = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  const int grid     = SPLIT ? tiles * plan.ways : (tiles < info->sm_count ? tiles : info->sm_count);
-  uint8_t*  ws       = SPLIT ? static_cast<uint8_t*>(registered_workspace(info->device).ptr) : nullptr;
-  float*    partials = SPLIT ? reinterpret_cast<float*>(ws + WS_HEADER_BYTES) : nullptr;
-  uint32_t* counters = SPLIT ? reinterpret_cast<uint32_t*>(ws + WS_RESERVED_BYTES) : nullptr;
+  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  const int grid  = SPLIT ? tiles * plan.ways : (tiles < info->sm_count ? tiles : info->sm_count);
   LLMMM_CUDA_TRY(launch_pdl(fp16_gemm_kernel<T, BN, SPLIT>, dim3(grid), dim3(THREADS), Fp16Layout<BN>::SMEM_BYTES, stream, 1, tm_a, tm_b,
-                            tm_c, M, N, K, plan.ways, plan.chunk, partials, counters, info->status));
+                            tm_c, M, N, K, plan.ways, plan.chunk, plan.partials, plan.counters, info->status));
   g_launches.fetch_add(1);
   return LLMMM_OK;
 }
