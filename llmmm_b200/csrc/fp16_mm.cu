@@ -779,7 +779,7 @@ struct Fp16Plan {
 // 64 / 128 / 256 wide.  A k-step of a 128x64 tile is 128 clk of MMAs, but 24 KB that one SM has to fetch.  Problems of one wave
 // took the pair kernel (cut along K if they were long) before they took narrow tiles: 256^3 5.5 -> 2.9 us, 512x1024x1024 9.0 ->
 // 4.7, 1001x1024x1544 11.9 -> 8.2, 512x2048x4096 22.8 -> 12.7; with the narrow tiles cut along K 256x256x4096 19.6 -> 8.7 (10.8
-// not cut), 300x1288x3592 21.7 -> 13.6; of up to 128 rows 16x4096x4096 22.5 -> 12.5, 128x12288x1024 10.7 -> 8.0.
+// not cut), 300x1288x3592 21.7 -> 13.6; of up to 128 rows 64x4096x4096 22.8 -> 11.6, 128x12288x1024 9.9 -> 6.1.
 static Fp16Plan fp16_plan(const DeviceInfo* info, int M, int N, int K, bool count)
 {
   const int       k_steps = (K + fp16cfg::BK - 1) / fp16cfg::BK;
@@ -798,6 +798,20 @@ static Fp16Plan fp16_plan(const DeviceInfo* info, int M, int N, int K, bool coun
   plan.ways  = 1;
   plan.chunk = k_steps;
   plan.bn    = tiles(64) <= info->sm_count ? 64 : tiles(128) <= info->sm_count ? 128 : 256;
+  // But TMA loads of an A below 128 KB take longer with every CTA that shares it, above all beyond half of the SMs (at 128 KB the
+  // effect is gone: 24x6144x2560 16.3 us, 28x6144x2560 8.3).  Where it decides, wider tiles are faster.  (With one or two k-steps
+  // it shows when A's rows begin inside sectors, with more if A is short or its rows do.)  Us with tiles 64 / 128 / 256 wide:
+  // 16x5120x1024 8.6 / 6.9 / 8.1, 12x9424x304 5.7 / 4.5 / 5.2, 54x5200x8 5.2 / 4.0 / 4.0, 1x7040x2224 17.8 / 15.4 / 13.5 (and where rows
+  // of B begin inside sectors, 1x8712x2224, 18.1 / 15.6 / 19.1), 15x10112x592 - / 8.6 / 7.3, 8x12288x4096 - / 33.1 / 28.5,
+  // 13x14528x1688 - / 17.6 / 18.6.
+  const int  half = info->sm_count / 2, third = info->sm_count / 3;
+  const bool odd  = K % 16 != 0;
+  if (M <= 128 && 2ll * M * K < 131072 && tiles(64) > half
+      && (k_steps >= 3 ? M < 64 || odd : k_steps == 2 ? odd : (odd || K < fp16cfg::BK) && M >= 16)) {
+    const bool wide = tiles(128) <= half ? tiles(128) > third && k_steps >= 20 && N % 32 == 0 :
+                                           tiles(256) < third && (k_steps >= 5 || (k_steps == 1 && odd));
+    plan.bn = wide || tiles(128) > info->sm_count ? 256 : 128;
+  }
   if (info->max_pairs < 1 || N <= 128 || M <= 64) {
     return plan;  // (calls of up to 64 rows never use scratch)
   }

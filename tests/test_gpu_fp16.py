@@ -198,3 +198,27 @@ def test_one_wave_of_narrow_tiles(capi, oracle, cuda, shape, dtype):
     for _ in range(2):  # (the second call finds the arrival counters as the first one left them)
         run_case(capi, oracle, cuda, M, N, K, dtype, seed=9, scratch=True)
     assert capi.split_launch_count() == n0 + (2 if ways > 1 else 0)
+
+
+# (M, N, K, tile width): A below 128 KB, where more CTAs make its loads slower: the edge at 128 KB, one k-step, rows of A that
+# begin inside sectors, and the edges at which the tiles get 128 and 256 wide.
+SMALL_A_SHAPES = [(24, 6144, 2560, 128), (26, 6144, 2560, 64), (16, 4736, 1024, 64), (16, 4744, 1024, 128), (63, 5120, 192, 128), (64, 5120, 192, 64),
+                  (16, 5120, 8, 128), (15, 5120, 8, 64), (100, 5120, 72, 128), (100, 5120, 96, 64), (6, 6688, 1688, 256), (6, 6680, 1688, 128),
+                  (5, 9472, 512, 128), (5, 9480, 512, 256), (5, 9480, 200, 128), (5, 12288, 264, 256), (5, 12296, 264, 128)]
+
+
+@pytest.mark.parametrize("shape", SMALL_A_SHAPES, ids=lambda s: "x".join(map(str, s[:3])))
+def test_tile_width_of_a_small_a(capi, oracle, cuda, shape):
+    M, N, K, width = shape
+    if torch.cuda.get_device_properties(cuda).multi_processor_count != 148:
+        pytest.skip("the tile width follows the number of SMs")
+    capi.clear_workspace()
+    assert f"tiles of 128x{width} " in capi.describe_plan("fp16", M, N, K)
+    run_case(capi, oracle, cuda, M, N, K, torch.float16, seed=10, scratch=False)
+
+
+def test_several_wide_tiles_per_cta(capi, oracle, cuda):
+    # 153 tiles of 128x256 on 148 CTAs: both accumulators of the single-CTA kernel
+    capi.clear_workspace()
+    assert "tiles of 128x256" in capi.describe_plan("bf16", 65, 38920, 72)
+    run_case(capi, oracle, cuda, 65, 38920, 72, torch.bfloat16, seed=11, scratch=False)
