@@ -774,12 +774,24 @@ struct Fp16Plan {
   uint32_t* counters;
 };
 
-// Times in ns, from a sweep of 19 shapes as launch chains (256..1333 x 256..4096 x 256..9728 and 1..128 rows): a pair kernel
-// takes 5400 and 280 per k-step of 64 and round of tiles, the single-CTA kernel 2900 and 153 / 200 / 270 per k-step for tiles
-// 64 / 128 / 256 wide.  A k-step of a 128x64 tile is 128 clk of MMAs, but 24 KB that one SM has to fetch.  Problems of one wave
-// took the pair kernel (cut along K if they were long) before they took narrow tiles: 256^3 5.5 -> 2.9 us, 512x1024x1024 9.0 ->
-// 4.7, 1001x1024x1544 11.9 -> 8.2, 512x2048x4096 22.8 -> 12.7; with the narrow tiles cut along K 256x256x4096 19.6 -> 8.7 (10.8
-// not cut), 300x1288x3592 21.7 -> 13.6; of up to 128 rows 64x4096x4096 22.8 -> 11.6, 128x12288x1024 9.9 -> 6.1.
+// What a row stride costs TMA loads: rows of a box that straddle two 128-byte lines, or also begin inside a 32-byte sector.
+static int stride_level(int elements)
+{
+  const int bytes = 2 * elements;
+  return bytes % 128 == 0 ? 0 : bytes % 64 == 0 ? 1 : bytes % 32 == 0 ? 3 : 10;
+}
+
+// Times in ns, from launch chains of some 200 shapes (129..6225 rows x 224..12288 x 256..9728).  A pair kernel takes 5400 and 280
+// per k-step of 64 and round of tiles; cutting the tiles of the last round in two costs 6000, in three 10700, in more 12500.  The
+// single-CTA kernel takes 2900 and per k-step 125 + tiles / 5 (tiles 64 wide: 128 clk of MMAs, but 24 KB that one SM has to fetch)
+// or 145 + 0.45 tiles (128 wide).  Strides cost per k-step and level of A / B 8.5 / 3.5 (64 wide), 5 / 5 (pair) and 13 / 9 (128 wide;
+// 40 more where both do, at most 200):
+// 256x1280x3584 10.4, 11.4 and (cut along K) 20.2 us, 256x1288x3592 18.8, 24.1 and 22.0.  (Without these terms long problems of
+// odd strides took 128-wide tiles where pairs cut along K are faster: 1333x1288x3592 25.7 us against 21.9, 6225x224x8464 38.0
+// against 33.2.)  Problems of one wave took the pair kernel (cut along K if they were long) before they took narrow tiles: 256^3
+// 5.5 -> 2.9 us, 512x1024x1024 9.0 -> 4.7, 1001x1024x1544 11.9 -> 8.2, 512x2048x4096 22.8 -> 12.7; with the narrow tiles cut along
+// K 256x256x4096 19.6 -> 8.7 (10.8 not cut), 300x1288x3592 21.7 -> 13.6; of up to 128 rows 64x4096x4096 22.8 -> 11.6,
+// 128x12288x1024 9.9 -> 6.1.
 static Fp16Plan fp16_plan(const DeviceInfo* info, int M, int N, int K, bool count)
 {
   const int       k_steps = (K + fp16cfg::BK - 1) / fp16cfg::BK;
@@ -816,39 +828,48 @@ static Fp16Plan fp16_plan(const DeviceInfo* info, int M, int N, int K, bool coun
     return plan;  // (calls of up to 64 rows never use scratch)
   }
   if (M <= 128) {
-    // 65..128 rows: the pair kernel if it cuts its few tiles along K
+    // 65..128 rows: the pair kernel if it cuts its few tiles along K (also where narrow tiles are faster: 128x4096x4096 22.6 against
+    // 11.9 us), or if A has many rows that begin inside sectors, K is long and tiles 64 wide are far from one wave (107x14080x3704
+    // 25.3 us against 28.2, 107x11000x8200 54.5 against 57.7; 80x14080x8200 47.2 against 45.7, 107x9728x8200 45.5 against 41.5)
     const SplitPlan sp = scratch && 2 * tiles(256) <= info->sm_count ? pair_plan(false) : SplitPlan{};
-    plan.pair          = sp.split_pairs > 0;
+    plan.pair          = sp.split_pairs > 0 || (sp.pairs > 0 && M > 80 && tiles(128) > half && k_steps >= 48 && odd);
     if (plan.pair) {
       plan.split = pair_plan(count);
     }
     return plan;
   }
+  const int lvl_a = stride_level(K), lvl_b = stride_level(N);
   long long narrow = -1;
   if (plan.bn < 256) {
-    narrow = 2900 + (plan.bn == 64 ? 153ll : 200ll) * k_steps;
+    int ways = 1, chunk = k_steps;
     if (plan.bn == 64 && scratch) {
+      long long best     = 2900 + 153ll * k_steps;
       const int max_ways = info->sm_count / tiles(64) < SPLIT_MAX_WAYS ? info->sm_count / tiles(64) : SPLIT_MAX_WAYS;
       for (int w = 2; w <= max_ways; ++w) {
         const int       c   = (k_steps + w - 1) / w;
         const long long est = 2900 + 153ll * c + 2000 + 300 * w;
-        if (est < narrow) {
-          narrow     = est;
-          plan.chunk = c;
-          plan.ways  = (k_steps + c - 1) / c;  // no empty chunks
+        if (est < best) {
+          best  = est;
+          chunk = c;
+          ways  = (k_steps + c - 1) / c;  // no empty chunks
         }
       }
     }
-  }
-  if (plan.ways > 1) {
-    // (the launch must not look the scratch up again: another thread may unregister or replace it meanwhile)
-    plan.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(ws.ptr) + WS_HEADER_BYTES);
-    plan.counters = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(ws.ptr) + WS_RESERVED_BYTES);
+    const int odd_128  = 13 * lvl_a + 9 * lvl_b + (lvl_a > 0 && lvl_b > 0 ? 40 : 0);
+    const int per_step = plan.bn == 64 ? 125 + tiles(64) / 5 + (17 * lvl_a + 7 * lvl_b) / 2 : 145 + tiles(128) * 9 / 20 + (odd_128 < 200 ? odd_128 : 200);
+    narrow             = 2900 + (long long)per_step * chunk + (ways > 1 ? 2000 + 300 * ways : 0);
+    plan.ways  = ways;
+    plan.chunk = chunk;
+    if (ways > 1) {
+      // (the launch must not look the scratch up again: another thread may unregister or replace it meanwhile)
+      plan.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(ws.ptr) + WS_HEADER_BYTES);
+      plan.counters = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(ws.ptr) + WS_RESERVED_BYTES);
+    }
   }
   const SplitPlan sp     = pair_plan(false);
   const long long rounds = sp.dp_tiles > 0 ? (sp.dp_tiles + sp.pairs - 1) / sp.pairs : 0;
-  const long long pair   = 5400 + 280 * (rounds * k_steps + (sp.split_pairs > 0 ? sp.split_chunk : 0))
-                         + (sp.split_pairs > 0 ? 3000 + 1500 * sp.split_s : 0);
+  const long long pair   = 5400 + (280 + 5 * (lvl_a + lvl_b)) * (rounds * k_steps + (sp.split_pairs > 0 ? sp.split_chunk : 0))
+                         + (sp.split_pairs == 0 ? 0 : sp.split_s == 2 ? 6000 : sp.split_s == 3 ? 10700 : 12500);
   plan.pair = narrow < 0 || pair < narrow;
   if (plan.pair) {
     plan.split = pair_plan(count);

@@ -222,3 +222,31 @@ def test_several_wide_tiles_per_cta(capi, oracle, cuda):
     capi.clear_workspace()
     assert "tiles of 128x256" in capi.describe_plan("bf16", 65, 38920, 72)
     run_case(capi, oracle, cuda, 65, 38920, 72, torch.bfloat16, seed=11, scratch=False)
+
+
+# Shapes whose last wave of 256x256 tiles is cut along K by the pair kernel, with M, N and K that no tile divides: rows that begin
+# inside sectors, where tiles 128 wide would be slower; whole waves of pairs before the cut tiles.
+PAIR_SPLIT_SHAPES = [(1333, 1288, 3592), (2310, 4360, 4104)]
+
+
+@pytest.mark.parametrize("shape", PAIR_SPLIT_SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_pair_kernel_cuts_ragged_tiles(capi, oracle, cuda, shape):
+    M, N, K = shape
+    if torch.cuda.get_device_properties(cuda).multi_processor_count != 148:
+        pytest.skip("which tiles are cut follows the number of SMs")
+    capi.ensure_workspace(M, N, K)
+    d = capi.describe_plan("bf16", M, N, K)
+    assert "fp16_gemm_pair_kernel" in d and "cut 2-way along K" in d
+    n0 = capi.split_launch_count()
+    run_case(capi, oracle, cuda, M, N, K, torch.bfloat16, seed=12, rows=[(0, 8), (250, 16), (M - 60, 60)], scratch=True)
+    # repeated calls agree bit for bit: the counters reset themselves and the chunks are added in a fixed order
+    g = torch.Generator(device=cuda).manual_seed(13)
+    A = torch.randn(M, K, device=cuda, generator=g).half()
+    B = torch.randn(K, N, device=cuda, generator=g).half()
+    outs = [torch.empty(M, N, dtype=torch.float16, device=cuda) for _ in range(4)]
+    for C in outs:
+        capi.fp16_mm(A, B, C, M, N, K)
+    torch.cuda.synchronize()
+    capi.check_status()
+    assert capi.split_launch_count() == n0 + 5
+    assert all(torch.equal(C, outs[0]) for C in outs[1:])
