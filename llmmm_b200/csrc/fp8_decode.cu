@@ -680,11 +680,12 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
     // Up to 16 columns warp 1 alone, else warps 1, 2 and 3 in turn; each K-block has its own ring slot and tensor-memory
     // partial stage, so the threads never touch the same barrier phase.  (One thread under elect.sync keeps up; with packed
     // FMAs beside it, layer at M = 1 / 16: 38.45 / 41.2 us with three threads, 38.2 / 40.9 with one; the GEMMs at M = 64
-    // 38.8 and 38.95 as a graph.)
-    constexpr int ISSUERS = MP <= 16 ? 1 : 3;
-    if (warp <= ISSUERS && elect_one()) {
+    // 38.8 and 38.95 as a graph.)  A cluster CTA whose run fits the ring takes three in any case: its K-blocks arrive together
+    // and one thread hands them on one after the other (7x2560x4096, four or five per CTA: 6.83 us with one, 6.65 with three).
+    const uint32_t issuers = MP > 16 || (CLUSTER && run <= (uint32_t)L::STAGES) ? 3u : 1u;
+    if ((uint32_t)warp <= issuers && elect_one()) {
       constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, 128, MP);
-      for (uint32_t it = (uint32_t)(warp - 1); it < run; it += ISSUERS) {
+      for (uint32_t it = (uint32_t)(warp - 1); it < run; it += issuers) {
         const uint32_t s  = it % L::STAGES;
         const uint32_t ph = (it / L::STAGES) & 1;
         mbar_wait(&bars->part_empty[s], ph ^ 1, DEV_WAIT_TMEM_EMPTY, abort_flag, status);

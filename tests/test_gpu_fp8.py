@@ -160,6 +160,20 @@ def test_qwen3_4b_decode_shapes(capi, oracle, cuda, M, NK):
     check_against_oracle(oracle, *case, gq, gs, gf)
 
 
+@pytest.mark.parametrize("M", [1, 16])
+@pytest.mark.parametrize("k_blocks", [7, 20, 42, 43, 49])
+def test_cluster_decode_around_the_ring_depth(capi, oracle, cuda, M, k_blocks):
+    # clusters of seven CTAs, one to seven K-blocks per CTA: up to the six of the ring three threads issue the MMAs, beyond it
+    # one; 43 K-blocks have both in one cluster
+    N, K = 2560, 128 * k_blocks
+    case = make_case(oracle, 51 + k_blocks, M, N, K)
+    gq, gs, gf = gpu_mm(capi, cuda, *case)
+    assert "clusters of 7 CTAs" in capi.describe_plan("fp8", M, N, K)
+    check_against_oracle(oracle, *case, gq, gs, gf)
+    gq2, gs2, gf2 = gpu_mm(capi, cuda, *case)
+    assert np.array_equal(gq, gq2) and np.array_equal(gs, gs2) and np.array_equal(gf, gf2)
+
+
 def test_decode_without_workspace_uses_general_kernel(capi, oracle, cuda):
     # no scratch registered -> the library must still compute (general kernel), never fail or fall back to a CPU
     case = make_case(oracle, 42, 16, 512, 1024)
