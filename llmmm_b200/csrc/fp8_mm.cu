@@ -43,8 +43,8 @@
 
 namespace llmmm {
 
-// Static weight tiles beyond the ring that the kernels for up to 128 rows request into L2 before the dependency wait: the four
-// GEMMs of a Qwen3-4B layer at 100 rows with none 48.5 us, four 48.6, eight 48.2, twelve and more 48.8.
+// Static weight tiles beyond the ring that go to L2 before the dependency wait of a call of up to 128 rows: the four GEMMs of a
+// Qwen3-4B layer at 100 rows with none 48.5 us, four 48.6, eight 48.2, twelve and more 48.8.
 constexpr int EARLY_L2 = 8;
 
 namespace fp8cfg {
@@ -1486,7 +1486,10 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
     setmaxnreg_dec<REGS_CTRL>();
     if (warp == 0) {
       // ---------------------------------------------------- TMA producer --
-      // (static weights: the first ring is requested before the dependency wait, as in the 256-row kernel)
+      // Static weights: the first ring is requested before the dependency wait, as in the 256-row kernel, unless the weight has
+      // fewer rows than the activations: then it is the smaller part, every row of tiles asks for it again, and the requests
+      // hold up the quantiser this kernel waits for (quantiser and GEMM, 1333x512x6144 20.4 us before early weights, 21.2 with
+      // them, 20.5 so; 768x512x6144 15.7, 16.2, 15.8; 129x6144x2560 11.4 without, 10.5 with).
       auto load_weights = [&](uint32_t s, int kb) {
         if (rank == 0) {
           mbar_arrive_expect_tx(&bars->full[s], STAGE_TX);
@@ -1494,12 +1497,15 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
         tma_load_2d_pair(smem + OFF_B + s * B_BYTES, &tm_b, mapa_shared(smem_u32(&bars->full[s]), leader), kb * BK,
                          SWIGLU ? tile * 128 + (int)rank * N : tile * BN + (int)rank * 128);
       };
-      const int early_end = early_weights ? min(kb0 + (int)STAGES, kb1) : kb0;
+      const bool early     = early_weights && (SWIGLU ? 2 * N : N) >= M;
+      const int  early_end = early ? min(kb0 + (int)STAGES, kb1) : kb0;
       if (elect_one()) {
         for (int kb = kb0; kb < early_end; ++kb) {
           load_weights((uint32_t)(kb - kb0), kb);
         }
-        if (early_weights) {  // (and the EARLY_L2 tiles behind the ring go to L2)
+        // The EARLY_L2 tiles behind the ring go to L2 if this is their only row of tiles (as one of several 192x4096x4096
+        // 14.06 us before, 14.6 with them, 14.2 without; 192x6144x2560 11.6, 11.6, 11.05).
+        if (early && m_tiles == 1) {
           for (int kb = early_end; kb < min(early_end + EARLY_L2, kb1); ++kb) {
             tma_prefetch_2d(&tm_b, kb * BK, SWIGLU ? tile * 128 + (int)rank * N : tile * BN + (int)rank * 128);
           }
