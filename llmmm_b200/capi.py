@@ -335,8 +335,8 @@ def tune(kind: str, N: int, K: int) -> None:
 
 def set_static_weights(enabled: bool) -> None:
     """Promise (or withdraw the promise) that the B operands of later FP8 GEMMs are weights that the kernel
-    running just before the GEMM on the same stream never writes; decode-sized calls then prefetch them while
-    that kernel is still finishing."""
+    running just before the GEMM on the same stream never writes; FP8 GEMMs of every size then read their first
+    weight tiles while that kernel is still finishing."""
     _check(lib().llmmm_set_static_weights(1 if enabled else 0))
 
 

@@ -1553,6 +1553,7 @@ __global__ void __launch_bounds__(fp8p128::THREADS, 1)
     }
     else if (rank == 0 && elect_one()) {
       // ------------------------------------ two MMA issuers (leader only) --
+      // (with one, e4m3 output takes 0 to 1.6 % longer)
       constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, BM, BN);
       const uint32_t     total = (uint32_t)(kb1 - kb0);
       for (uint32_t it = warp == 1 ? 0u : 1u; it < total; it += 2) {
