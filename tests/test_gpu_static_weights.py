@@ -4,6 +4,8 @@ not.  The weight quantiser runs before that quantiser.  Results equal those of c
 import pytest
 import torch
 
+from llmmm_b200.host_pipeline import Fp8GemmHostPipeline
+
 pytestmark = pytest.mark.gpu
 
 # (form, M, columns of the output, K): the 128-row and the 256-row kernel, K shorter and longer than their rings, a ragged last row
@@ -55,3 +57,34 @@ def test_early_weights_change_nothing(capi, cuda, case):
     finally:
         capi.set_static_weights(False)
     capi.check_status()
+
+
+@pytest.mark.parametrize("shape", [(16, 2560, 4096), (100, 2560, 4096), (1000, 9600, 1024)], ids=lambda s: "x".join(map(str, s)))
+def test_weights_copied_from_the_host_before_every_call(capi, cuda, shape):
+    # the copies run on another stream and are waited for by an event: the next kernel must not start, and read, before them
+    M, N, K = shape
+    g = torch.Generator(device=cuda).manual_seed(67)
+    calls = []
+    for i in range(6):
+        A_q, A_s = torch.empty(M, K, dtype=torch.uint8, device=cuda), torch.empty(K // 128, M, device=cuda)
+        B_q, B_s = torch.empty(N, K, dtype=torch.uint8, device=cuda), torch.empty(N // 128, K // 128, device=cuda)
+        capi.fp8_quant_1x128(torch.randn(M, K, device=cuda, generator=g), A_q, A_s, M, K)
+        capi.fp8_quant_128x128(torch.randn(N, K, device=cuda, generator=g), B_q, B_s, N, K)
+        calls.append((A_q, A_s, B_q, B_s))
+    pipe = Fp8GemmHostPipeline(M, N, K, depth=2, device=cuda)
+    expected = []
+    for ops in calls:
+        C_q, C_s = torch.empty(M, N, dtype=torch.uint8, device=cuda), torch.empty(N // 128, M, device=cuda)
+        capi.fp8_blockwise_mm(*ops, C_q, C_s, M, N, K)
+        expected.append((C_q.cpu(), C_s.cpu()))
+    host = [[t.cpu().pin_memory() for t in ops] for ops in calls]
+    results = [(torch.empty(M, N, dtype=torch.uint8).pin_memory(), torch.empty(N // 128, M).pin_memory()) for _ in calls]
+    capi.set_static_weights(True)
+    try:
+        for ops, out in zip(host, results):
+            pipe.submit(*ops, *out)
+        pipe.drain()
+    finally:
+        capi.set_static_weights(False)
+    for got, want in zip(results, expected):
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
