@@ -16,7 +16,7 @@
 //     groups, and only the left-over groups are cut evenly among the CTAs,
 //     which work on those cut pieces FIRST;
 //   * warp 0 streams weight blocks (and the matching activation slab) through
-//     a 6-8-deep TMA ring; warp 1 (32 and 64 columns: warps 1-3 in turn) issues
+//     a 6-8-deep TMA ring; warp 1 (cluster kernel: 1-2, 32 and 64 columns: 1-3 in turn) issues
 //     the MMAs of a K-block (four per K-block, from zero, into the tensor-memory
 //     partial stage of the ring slot); the promotion warps (4, or 8 for 32 and 64 columns) promote
 //     with acc = fma(partial, A_s*B_s, acc) in registers, the scale products of
@@ -52,7 +52,7 @@ namespace deccfg {
 constexpr int      BK            = 128;
 constexpr int      UMMA_K        = 32;
 constexpr int      MAX_STAGES    = 8;    // the ring depth depends on the activation tile, see DecodeSmem
-// warps 0-3: producer, one or three MMA issuers; warps 4-7 (up to 16 activation columns) or 4-11 (32, 64 columns): promotion.
+// warps 0-3: producer, one to three MMA issuers; warps 4-7 (up to 16 activation columns) or 4-11 (32, 64 columns): promotion.
 // With 64 columns one promotion warp per scheduler could not keep up with the weight stream (measured: ~600 ns per
 // K-block, all of it latency: shared-memory loads, the barrier, tensor-memory loads, 64 FMAs, one after the other
 // with nothing to overlap; HBM delivers a block every 364 ns): two warps per scheduler take half of the columns
@@ -677,15 +677,16 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
   }
   else if (warp < EPI_WARP0) {
     // --------------------------------------------- MMA issuers ------------
-    // Up to 16 columns warp 1 alone, else warps 1, 2 and 3 in turn; each K-block has its own ring slot and tensor-memory
-    // partial stage, so the threads never touch the same barrier phase.  (One thread under elect.sync keeps up; with packed
-    // FMAs beside it, layer at M = 1 / 16: 38.45 / 41.2 us with three threads, 38.2 / 40.9 with one; the GEMMs at M = 64
-    // 38.8 and 38.95 as a graph.)  A cluster CTA whose run fits the ring takes three in any case: its K-blocks arrive together
-    // and one thread hands them on one after the other (7x2560x4096, four or five per CTA: 6.83 us with one, 6.65 with three).
-    const uint32_t issuers = MP > 16 || (CLUSTER && run <= (uint32_t)L::STAGES) ? 3u : 1u;
-    if ((uint32_t)warp <= issuers && elect_one()) {
+    // Up to 16 columns warp 1 alone, in the cluster kernel warps 1 and 2, with more columns warps 1, 2 and 3 in turn; each
+    // K-block has its own ring slot and tensor-memory partial stage, so the threads never touch the same barrier phase.  One
+    // thread under elect.sync keeps up with a stream; a cluster CTA has few K-blocks, which arrive together.  (Cluster kernels
+    // with one, two, three threads: layer at M = 1 / 16 37.96 / 40.78, 37.84 / 40.68, 38.2 / 41.0 us; without static weights
+    // 7x2560x4096 after its quantiser 6.88, 6.70, 6.67.  Stream kernels up to 16 columns as a graph, one and three threads: 38.2 and
+    // 38.45 us a layer at M = 1.  Four GEMMs at M = 64 as a graph: 38.95 with one, 38.8 with three.)
+    constexpr int ISSUERS = MP > 16 ? 3 : CLUSTER ? 2 : 1;
+    if (warp <= ISSUERS && elect_one()) {
       constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, 128, MP);
-      for (uint32_t it = (uint32_t)(warp - 1); it < run; it += issuers) {
+      for (uint32_t it = (uint32_t)(warp - 1); it < run; it += ISSUERS) {
         const uint32_t s  = it % L::STAGES;
         const uint32_t ph = (it / L::STAGES) & 1;
         mbar_wait(&bars->part_empty[s], ph ^ 1, DEV_WAIT_TMEM_EMPTY, abort_flag, status);

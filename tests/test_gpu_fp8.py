@@ -165,8 +165,8 @@ def test_qwen3_4b_decode_shapes(capi, oracle, cuda, M, NK):
 @pytest.mark.parametrize("M", [1, 16])
 @pytest.mark.parametrize("run", [(1, 0), (3, 2), (6, 0), (6, 1), (7, 0)], ids=lambda r: f"{r[0]}+{r[1]}")
 def test_cluster_decode_around_the_ring_depth(capi, oracle, cuda, M, run):
-    # one to seven K-blocks per CTA of a cluster: up to the six of the ring three threads issue the MMAs, beyond it one;
-    # (6, 1) has both in one cluster.  (How many CTAs a cluster has follows how many clusters the device holds.)
+    # one to seven K-blocks per CTA of a cluster, whose MMAs two threads issue in turn: odd and even runs, the six of the ring
+    # and one more, in all CTAs of a cluster or in one.  (How many CTAs it has follows how many clusters the device holds.)
     N = 2560
     size = int(re.search(r"clusters of (\d) CTAs", capi.describe_plan("fp8", M, N, 4096))[1])
     K = 128 * (size * run[0] + run[1])
