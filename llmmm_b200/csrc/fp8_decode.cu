@@ -679,10 +679,10 @@ __global__ void __launch_bounds__(deccfg::threads(MP, CLUSTER), deccfg::ctas_per
     // --------------------------------------------- MMA issuers ------------
     // Up to 16 columns warp 1 alone, in the cluster kernel warps 1 and 2, with more columns warps 1, 2 and 3 in turn; each
     // K-block has its own ring slot and tensor-memory partial stage, so the threads never touch the same barrier phase.  One
-    // thread under elect.sync keeps up with a stream; a cluster CTA has few K-blocks, which arrive together.  (Cluster kernels
-    // with one, two, three threads: layer at M = 1 / 16 37.96 / 40.78, 37.84 / 40.68, 38.2 / 41.0 us; without static weights
-    // 7x2560x4096 after its quantiser 6.88, 6.70, 6.67.  Stream kernels up to 16 columns as a graph, one and three threads: 38.2 and
-    // 38.45 us a layer at M = 1.  Four GEMMs at M = 64 as a graph: 38.95 with one, 38.8 with three.)
+    // thread under elect.sync keeps up with a stream; a cluster CTA has few K-blocks, which arrive together.  (Layer at M = 1 / 16:
+    // 38.45 / 41.2 us with three threads in all kernels, 38.2 / 40.9 with one; later 37.96 / 40.78 with one, 37.84 / 40.68 with two in the
+    // cluster kernel.  Without static weights 7x2560x4096 after its quantiser 6.88 us with one thread, 6.70 with two, 6.67 with three.
+    // Four GEMMs at M = 64 as a graph: 38.95 with one, 38.8 with three.)
     constexpr int ISSUERS = MP > 16 ? 3 : CLUSTER ? 2 : 1;
     if (warp <= ISSUERS && elect_one()) {
       constexpr uint32_t idesc = make_idesc(/*e4m3*/ 0, 0, 0, 0, 128, MP);
